@@ -46,7 +46,10 @@ constexpr int kMaxChunk = 32;
 constexpr int kDefaultChunk = 16;   // ranks per k_step CTA when nothing else decides
 constexpr int kMaxChunks = kMaxBeam / kMinChunk;
 static_assert(kMinChunk % kWarpsPerStepCta == 0 && kMaxChunk <= 32, "a chunk is 1..4 ranks per warp");
-constexpr int kSelectThreads = 1024;
+#ifndef BSJ_SELECT_THREADS
+#define BSJ_SELECT_THREADS 1024
+#endif
+constexpr int kSelectThreads = BSJ_SELECT_THREADS;   // block size of the one-block selection routes
 constexpr int kHeapThreads = 256;    // k_heap: warp 0 runs the heap, warps 1..7 prepare chunks
 constexpr int kHeapMaxChunk = 32;     // parents per k_heap chunk (at most)
 
@@ -171,6 +174,15 @@ __device__ __forceinline__ uint16_t* H_NS(uint8_t* b, const Lay& L) { return rei
 __device__ __forceinline__ int32_t* H_CMAX(uint8_t* b, const Lay& L) { return reinterpret_cast<int32_t*>(b + L.off_hdr + 4); }
 __device__ __forceinline__ uint32_t* H_LIN(uint8_t* b, const Lay& L) { return reinterpret_cast<uint32_t*>(b + L.off_hdr + 8); }
 __device__ __forceinline__ uint32_t* H_STAMP(uint8_t* b, const Lay& L) { return reinterpret_cast<uint32_t*>(b + L.off_hdr + 12); }
+
+// Asynchronous 16-byte copies, global (L2) to shared memory.
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
+{
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem_dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem_src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
 // Warp-cooperative 16-byte copies (sbytes is a multiple of 16, buffers 16-byte aligned).
 __device__ __forceinline__ void warp_load(uint8_t* dst_smem, const uint8_t* src_gmem, int sbytes, int lane)

@@ -14,6 +14,7 @@
 // memory allocated once per call (gpu/v1/solver.cu:178-298, gpu/v2_twophases/solver.cu:
 // 256-386).  The whole sequence is captured once into a CUDA graph and replayed.
 #include <algorithm>
+#include <array>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -38,6 +39,7 @@ struct bsj_context {
     std::string err;
     int sm_count = 0;
     int max_smem_optin = 0;
+    SearchDevice search;    // what the device offers the resident search
     // plans of recent batch shapes (most recent last), reused with new data
     std::vector<std::pair<std::string, bsj_plan*>> cache;
     uint64_t hits = 0;
@@ -75,7 +77,17 @@ struct bsj_plan {
         int64_t knmax_gpu = 0;   // largest K * n of its gpu-mode beams (4 CTAs per beam from
                                  // kSelectClusterWideKN on)
     };
-    std::vector<Group> groups;
+    std::vector<Group> groups;        // all beams, for the level kernels (forced forms and routes)
+    std::vector<Group> rest_groups;   // the beams the resident search does not take
+    // resident search (bsj_search.cu): launches of [0] the rule's blocks per beam, [1] at most
+    // kSearchNarrow of them (bsj_plan_set_select_cluster)
+    struct Search {
+        SearchCfg cf{};
+        int nbeams = 0;
+        bool v1 = false;
+    };
+    std::vector<Search> search[2];
+    int nrest = 0;                    // segments [0, nrest) are not resident-search beams
     cudaEvent_t fork = nullptr;
     cudaEvent_t join[kMaxBranches] = {};
     std::vector<SegDesc> segs;
@@ -258,6 +270,133 @@ int rule_chunk_var(int64_t ranks, int nq, int64_t granks, bool group_ok, int kma
     return chunk_var_of((nq == 4 || granks > 8192) ? 32 : 16);
 }
 
+// Estimated makespan (us) of the resident searches with blocks[i] blocks each, started
+// longest first as the device's SMs allow.
+double search_makespan(const std::vector<double>& us, const std::vector<int>& blocks, int sms)
+{
+    std::vector<int> order(us.size());
+    for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return us[x] > us[y]; });
+    std::vector<std::pair<double, int>> running;   // min-heap of (end, blocks)
+    auto later = [](const std::pair<double, int>& x, const std::pair<double, int>& y) { return x.first > y.first; };
+    double now = 0, end = 0;
+    int free = sms;
+    for (int i : order) {
+        while (free < blocks[i] && !running.empty()) {
+            std::pop_heap(running.begin(), running.end(), later);
+            now = std::max(now, running.back().first);
+            free += running.back().second;
+            running.pop_back();
+        }
+        free -= blocks[i];
+        running.push_back({now + us[i], blocks[i]});
+        std::push_heap(running.begin(), running.end(), later);
+        end = std::max(end, now + us[i]);
+    }
+    return end;
+}
+
+// Blocks per beam of the plan's resident searches: for each largest size, every beam at its
+// fastest, or only as wide as finishing within 1, 1.5, 2 or 3 times the longest search needs;
+// the choice with the smallest estimated makespan.  (Few beams end up wide, a batch's short
+// searches narrow.)
+std::vector<int> search_shares(const bsj_plan* p, int cmax_form)
+{
+    const SearchDevice& dev = p->ctx->search;
+    const int count = p->nseg - p->nrest;
+    constexpr int kSizes = sizeof(kSearchSizes) / sizeof(kSearchSizes[0]);
+    struct Choice { int c; double us; };
+    std::vector<std::array<Choice, kSizes>> upto(count);   // [beam][largest size]
+    for (int i = 0; i < count; i++) {
+        const SegDesc& d = p->segs[p->nrest + i];
+        const bool v1 = d.mode == BSJ_MODE_V1;
+        for (int k = 0; k < kSizes; k++) {
+            const int c = search_blocks(dev, d.n, d.m, d.K, v1, kSearchSizes[k]);
+            upto[i][k] = Choice{c, d.N * search_level_us(d.n, d.K, v1, c)};
+        }
+    }
+    std::vector<int> best, c(count);
+    std::vector<double> us(count);
+    double best_us = 0;
+    for (int k = 0; k < kSizes && kSearchSizes[k] <= cmax_form; k++) {
+        if (dev.clusters[kSearchSizes[k]] < 1) continue;
+        double longest = 0;
+        for (int i = 0; i < count; i++) longest = std::max(longest, upto[i][k].us);
+        for (double slack : {0.0, 1.0, 1.5, 2.0, 3.0}) {
+            int most = 1;
+            for (int i = 0; i < count; i++) {
+                int w = k;
+                if (slack > 0)
+                    for (int q = 0; q < k; q++)
+                        if (upto[i][q].us <= slack * longest) { w = q; break; }
+                c[i] = upto[i][w].c;
+                us[i] = upto[i][w].us;
+                most = std::max(most, c[i]);
+            }
+            const double t = search_makespan(us, c, dev.clusters[most] * most);
+            if (best.empty() || t < best_us) { best = c; best_us = t; }
+        }
+    }
+    return best;
+}
+
+// The plan's resident-search launches: beams sharing a block count, lane count and mode
+// class run in one launch, longest search first.
+void plan_searches(bsj_plan* p, std::vector<int32_t>& list, int32_t* d_list, unsigned long long* spill)
+{
+    const SearchDevice& dev = p->ctx->search;
+    for (int form = 0; form < 2; form++) {
+        struct Class { int c, lanes, kmax, nmax, opsmax, smax; bool v1; double us; std::vector<int32_t> segs; };
+        std::vector<Class> classes;
+        const std::vector<int> share = search_shares(p, form == 0 ? kSearchMaxCluster : kSearchNarrow);
+        for (int si = p->nrest; si < p->nseg; si++) {
+            const SegDesc& d = p->segs[si];
+            const int S = SearchLay(d.n, d.m).bytes, c = share[si - p->nrest], lanes = search_lanes(d.n, d.K, c);
+            const bool v1 = d.mode == BSJ_MODE_V1;
+            const double us = d.N * search_level_us(d.n, d.K, v1, c);
+            // a launch lays its shared memory out for its largest beam: a beam joins a class only
+            // where that costs neither of them survivors per round
+            auto fits = [&](const Class& x) {
+                if (x.c != c || x.lanes != lanes || x.v1 != v1) return false;
+                SearchCfg both, one, other;
+                search_layout(one, c, lanes, d.K, d.n, d.N, S, dev.smem);
+                search_layout(other, c, lanes, x.kmax, x.nmax, x.opsmax, x.smax, dev.smem);
+                return search_layout(both, c, lanes, std::max(x.kmax, d.K), std::max(x.nmax, d.n),
+                                     std::max(x.opsmax, d.N), std::max(x.smax, S), dev.smem) &&
+                       both.rs == one.rs && both.rs == other.rs;
+            };
+            auto it = std::find_if(classes.begin(), classes.end(), fits);
+            if (it == classes.end()) {
+                classes.push_back(Class{c, lanes, d.K, d.n, d.N, S, v1, us, {si}});
+            } else {
+                it->kmax = std::max(it->kmax, d.K);
+                it->nmax = std::max(it->nmax, d.n);
+                it->opsmax = std::max(it->opsmax, d.N);
+                it->smax = std::max(it->smax, S);
+                it->us = std::max(it->us, us);
+                it->segs.push_back(si);
+            }
+        }
+        std::stable_sort(classes.begin(), classes.end(), [](const Class& x, const Class& y) { return x.us > y.us; });
+        size_t at = (size_t)form * p->nseg;
+        for (Class& x : classes) {
+            auto us = [&](int32_t si) {
+                return p->segs[si].N * search_level_us(p->segs[si].n, p->segs[si].K, x.v1, x.c);
+            };
+            std::stable_sort(x.segs.begin(), x.segs.end(), [&](int32_t a, int32_t b) { return us(a) > us(b); });
+            bsj_plan::Search sr;
+            search_layout(sr.cf, x.c, x.lanes, x.kmax, x.nmax, x.opsmax, x.smax, dev.smem);
+            sr.cf.list = d_list + at;
+            sr.cf.spill = spill;
+            sr.cf.wide = form == 0 ? 1 : 0;
+            sr.nbeams = (int)x.segs.size();
+            sr.v1 = x.v1;
+            for (int32_t si : x.segs) list[at++] = si;
+            p->search[form].push_back(sr);
+        }
+    }
+}
+
 // With `bytes_only` non-null, computes the plan's device footprint into it and allocates
 // nothing (*out is left untouched).
 bsj_status plan_build(bsj_context* ctx, int ninst, const bsj_instance* insts, int nbeams,
@@ -308,7 +447,22 @@ bsj_status plan_build(bsj_context* ctx, int ninst, const bsj_instance* insts, in
         const int i = beams[b].instance;
         return (i >= 0 && i < ninst) ? insts[i].n * insts[i].m : 0;
     };
-    std::stable_sort(p->perm.begin(), p->perm.end(), [&](int x, int y) { return levels_of(x) > levels_of(y); });
+    // beams the resident search does not take come first (they form the level kernels' groups)
+    std::vector<char> is_resident(nbeams, 0);
+    auto resident = [&](int b) { return is_resident[b] != 0; };
+    auto takes = [&](int b) {
+        const int i = beams[b].instance;
+        return beams[b].mode >= BSJ_MODE_V1 && beams[b].mode <= BSJ_MODE_CLEAN && i >= 0 && i < ninst &&
+               insts[i].m >= 2 && beams[b].beam_width >= 1 && beams[b].beam_width <= BSJ_MAX_BEAM &&
+               search_blocks(ctx->search, insts[i].n, insts[i].m, beams[b].beam_width,
+                             beams[b].mode == BSJ_MODE_V1, kSearchMaxCluster) > 0;
+    };
+    for (int b = 0; b < nbeams; b++) is_resident[b] = takes(b) ? 1 : 0;
+    std::stable_sort(p->perm.begin(), p->perm.end(), [&](int x, int y) {
+        if (resident(x) != resident(y)) return !resident(x);
+        return levels_of(x) > levels_of(y);
+    });
+    while (p->nrest < nbeams && !resident(p->perm[p->nrest])) p->nrest++;
 
     // per-beam layout
     size_t off_beam = 0, off_slot = 0, off_keys = 0, off_sel = 0, off_mask = 0, off_hist = 0, off_kcnt = 0,
@@ -343,12 +497,14 @@ bsj_status plan_build(bsj_context* ctx, int ninst, const bsj_instance* insts, in
         off_kcnt += (d.K + kMinChunk - 1) / kMinChunk;
         const size_t K = (size_t)d.K, n = (size_t)d.n, N = (size_t)d.N;
         const bool gpu = d.mode <= BSJ_MODE_CLEAN;
+        // room for a snapshot of either layout (level kernels / resident search)
+        const size_t snap = gpu ? (size_t)std::max(d.sbytes, SearchLay(d.n, d.m).bytes) : (size_t)d.sbytes;
         const int nbuf = (d.mode == BSJ_MODE_V1) ? 1 : 2;
         d.beam_off[0] = (int64_t)off_beam;
-        d.beam_off[1] = (int64_t)(off_beam + (nbuf == 2 ? align_up(K * d.sbytes, 256) : 0));
-        off_beam += nbuf * align_up(K * d.sbytes, 256);
+        d.beam_off[1] = (int64_t)(off_beam + (nbuf == 2 ? align_up(K * snap, 256) : 0));
+        off_beam += nbuf * align_up(K * snap, 256);
         d.slot_off = (int64_t)off_slot;
-        if (d.mode == BSJ_MODE_V1) off_slot += align_up(K * n * d.sbytes, 256);
+        if (d.mode == BSJ_MODE_V1) off_slot += align_up(K * n * snap, 256);
         d.key_off = (int64_t)off_keys;
         if (gpu) off_keys += align_up((size_t)((d.K + kMaxChunk - 1) / kMaxChunk) * kMaxChunk * n, 32);
         d.sel_off = (int64_t)off_sel;
@@ -428,6 +584,8 @@ bsj_status plan_build(bsj_context* ctx, int ninst, const bsj_instance* insts, in
     const size_t o_beam = take(off_beam);
     const size_t o_slot = take(off_slot);
     const size_t o_keys = take(8 * off_keys);
+    const size_t o_spill = take(p->nrest < nbeams ? 8 * off_keys : 0);
+    const size_t o_slist = take(2 * sizeof(int32_t) * nbeams);
     const size_t o_sel = take(4 * off_sel);
     const size_t o_mask = take(4 * off_mask);
     const size_t o_hist = take(4 * off_hist);
@@ -486,6 +644,10 @@ bsj_status plan_build(bsj_context* ctx, int ninst, const bsj_instance* insts, in
     a.noise = reinterpret_cast<const float*>(base + o_noise);
     a.dnoise = reinterpret_cast<const double*>(base + o_dnoise);
 
+    std::vector<int32_t> slist(2 * (size_t)nbeams, 0);
+    plan_searches(p, slist, reinterpret_cast<int32_t*>(base + o_slist),
+                  reinterpret_cast<unsigned long long*>(base + o_spill));
+
     // uploads (synchronous: the host vectors are pageable)
     cudaStream_t st = ctx->stream;
     cudaError_t e = cudaSuccess;
@@ -496,6 +658,7 @@ bsj_status plan_build(bsj_context* ctx, int ninst, const bsj_instance* insts, in
         e = cudaMemcpyAsync(p->d_cprefix + (size_t)v * (nbeams + 1), p->cprefix[v].data(), sizeof(int32_t) * (nbeams + 1),
                             cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(p->d_group_init, p->group_init.data(), sizeof(int32_t) * p->ngroups, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(base + o_slist, slist.data(), sizeof(int32_t) * slist.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(base + o_ops, ops.data(), sizeof(uint32_t) * ops.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = launch_noise_table(reinterpret_cast<float*>(base + o_noise),
                                                         reinterpret_cast<double*>(base + o_dnoise), st);
@@ -516,27 +679,27 @@ bsj_status plan_build(bsj_context* ctx, int ninst, const bsj_instance* insts, in
     p->gather_grid = std::max(1, std::min(want, ctx->sm_count * 8));
     // beam groups, balanced by work (K * levels); BSJ_MAX_BEAM_GROUPS in the environment
     // lowers the number of concurrent groups (1 = all beams in lockstep, for measurements)
-    {
+    auto make_groups = [&](int first, int end, std::vector<bsj_plan::Group>& out_groups) {
         int gmax = kMaxBranches;
         if (const char* env = std::getenv("BSJ_MAX_BEAM_GROUPS")) {
             const int v = std::atoi(env);
             if (v >= 1 && v < gmax) gmax = v;
         }
-        const int G = std::min(nbeams, gmax);
+        const int G = std::min(end - first, gmax);
         double total = 0;
-        for (int b = 0; b < nbeams; b++) total += (double)p->segs[b].K * p->segs[b].N;
-        int lo = 0;
+        for (int b = first; b < end; b++) total += (double)p->segs[b].K * p->segs[b].N;
+        int lo = first;
         double acc = 0;
-        for (int g = 0; g < G && lo < nbeams; g++) {
+        for (int g = 0; g < G && lo < end; g++) {
             int hi = lo + 1;
             acc += (double)p->segs[lo].K * p->segs[lo].N;
             const double target = total * (g + 1) / G;
-            while (hi < nbeams && (nbeams - hi) > (G - 1 - g) && acc + 0.5 * (double)p->segs[hi].K * p->segs[hi].N <= target) {
+            while (hi < end && (end - hi) > (G - 1 - g) && acc + 0.5 * (double)p->segs[hi].K * p->segs[hi].N <= target) {
                 acc += (double)p->segs[hi].K * p->segs[hi].N;
                 hi++;
             }
             if (g == G - 1) {
-                while (hi < nbeams) { acc += (double)p->segs[hi].K * p->segs[hi].N; hi++; }
+                while (hi < end) { acc += (double)p->segs[hi].K * p->segs[hi].N; hi++; }
             }
             bsj_plan::Group gr;
             gr.args = p->args;
@@ -552,7 +715,6 @@ bsj_status plan_build(bsj_context* ctx, int ninst, const bsj_instance* insts, in
                 if (d.mode == BSJ_MODE_V1) gr.has_v1 = true;
                 if (d.mode <= BSJ_MODE_CLEAN) {
                     gr.has_gpu = true;
-                    if (d.K >= kSelectClusterMinK) p->cluster_beams++;
                     gr.kmax_gpu = std::max(gr.kmax_gpu, d.K);
                     gr.knmax_gpu = std::max(gr.knmax_gpu, (int64_t)d.K * d.n);
                 } else {
@@ -568,18 +730,25 @@ bsj_status plan_build(bsj_context* ctx, int ninst, const bsj_instance* insts, in
             }
             const int wr = (p->prefix[hi] - p->prefix[lo] + kWarpsPerStepCta - 1) / kWarpsPerStepCta;
             gr.gather_grid = std::max(1, std::min(wr, ctx->sm_count * 8));
-            if (gr.has_gpu && gr.kmax_gpu >= kSelectClusterMinK) p->cluster_matters = true;
-            p->groups.push_back(gr);
+            out_groups.push_back(gr);
             lo = hi;
         }
-        // too many wide beams for even 2 CTAs each: the select form cannot differ
-        if ((int64_t)p->cluster_beams * 2 > ctx->sm_count) p->cluster_matters = false;
-        cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming);
-        for (int g = 0; g < (int)p->groups.size(); g++) cudaEventCreateWithFlags(&p->join[g], cudaEventDisableTiming);
-    }
+    };
+    make_groups(0, nbeams, p->groups);
+    if (p->nrest > 0) make_groups(0, p->nrest, p->rest_groups);
+    for (const SegDesc& d : p->segs)
+        if (d.mode <= BSJ_MODE_CLEAN && d.K >= kSelectClusterMinK) p->cluster_beams++;
+    // the select form differs where the resident search gives some beam several blocks, or the
+    // level kernels' cluster select applies (too many wide beams for even 2 CTAs each: not)
+    p->cluster_matters = p->cluster_beams > 0 && (int64_t)p->cluster_beams * 2 <= ctx->sm_count;
+    for (const auto& sr : p->search[0])
+        if (sr.cf.cluster > kSearchNarrow) p->cluster_matters = true;
+    cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming);
+    for (cudaEvent_t& ev : p->join) cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
     // chunk sizes: the default rule per group; the variant tuning found for this shape on
     // this device, else the rule
-    for (auto& gr : p->groups) {
+    for (auto* gv : {&p->groups, &p->rest_groups})
+    for (auto& gr : *gv) {
         int64_t per_nq[5] = {0, 0, 0, 0, 0};
         for (int b = gr.args.seg_lo; b < gr.args.seg_hi; b++) per_nq[p->segs[b].nq] += p->segs[b].K;
         const int nq = per_nq[4] > per_nq[2] && per_nq[4] > per_nq[1] ? 4 : (per_nq[2] > per_nq[1] ? 2 : 1);
@@ -638,6 +807,10 @@ cudaEvent_t* next_events(bsj_plan* p, int cls)
     ev.first = cls;
     return &ev.second.first;
 }
+
+// The resident search runs the plan's gpu-mode beams unless a k_step form or a selection
+// route is forced.
+bool uses_search(const bsj_plan* p) { return p->variant == 0 && p->select_force == 0; }
 
 // Enqueue one run of the plan on `s` (`capturing`: s is being captured into a graph, so
 // timing events become event-record nodes of the graph).
@@ -711,21 +884,43 @@ cudaError_t enqueue_run(bsj_plan* p, cudaStream_t s, bool capturing)
         }
         return cudaSuccess;
     };
-    if (p->groups.size() <= 1) {
-        e = group_loop(p->groups[0], s);
+    // independent parts: the resident-search launches and the level kernels' beam groups
+    const bool res = uses_search(p);
+    const auto& searches = p->search[p->select_cluster ? 0 : 1];
+    const auto& groups = res ? p->rest_groups : p->groups;
+    const size_t nsearch = res ? searches.size() : 0, parts = nsearch + groups.size();
+    auto run_part = [&](size_t i, cudaStream_t gs) -> cudaError_t {
+        if (i >= nsearch) return group_loop(groups[i - nsearch], gs);
+        const bsj_plan::Search& sr = searches[i];
+        if (!p->timing) { p->launches++; return launch_search(p->args, sr.cf, sr.nbeams, sr.v1, gs); }
+        cudaEvent_t* ev = next_events(p, 5);
+        auto rec = [&](cudaEvent_t x) {
+            return capturing ? cudaEventRecordWithFlags(x, gs, cudaEventRecordExternal) : cudaEventRecord(x, gs);
+        };
+        cudaError_t r = rec(ev[0]);
+        if (r == cudaSuccess) r = launch_search(p->args, sr.cf, sr.nbeams, sr.v1, gs);
+        if (r != cudaSuccess) return r;
+        p->launches++;
+        return rec(ev[1]);
+    };
+    if (parts == 1) {
+        e = run_part(0, s);
         if (e != cudaSuccess) return e;
     } else {
         e = cudaEventRecord(p->fork, s);
         if (e != cudaSuccess) return e;
-        for (size_t g = 0; g < p->groups.size(); g++) {
-            cudaStream_t gs = p->ctx->branch[g];
-            e = cudaStreamWaitEvent(gs, p->fork, 0);
+        const size_t used = std::min(parts, (size_t)kMaxBranches);
+        for (size_t g = 0; g < used; g++) {
+            e = cudaStreamWaitEvent(p->ctx->branch[g], p->fork, 0);
             if (e != cudaSuccess) return e;
-            e = group_loop(p->groups[g], gs);
+        }
+        for (size_t i = 0; i < parts; i++) {
+            e = run_part(i, p->ctx->branch[i % kMaxBranches]);
             if (e != cudaSuccess) return e;
-            e = cudaEventRecord(p->join[g], gs);
-            if (e != cudaSuccess) return e;
-            e = cudaStreamWaitEvent(s, p->join[g], 0);
+        }
+        for (size_t g = 0; g < used; g++) {
+            e = cudaEventRecord(p->join[g], p->ctx->branch[g]);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(s, p->join[g], 0);
             if (e != cudaSuccess) return e;
         }
     }
@@ -920,6 +1115,8 @@ bsj_status bsj_create(bsj_context** out, int device)
         e = cudaStreamCreateWithFlags(&ctx->branch[g], cudaStreamNonBlocking);
     if (e != cudaSuccess) { delete ctx; return BSJ_ERR_CUDA; }
     ctx->device = device;
+    e = search_device(ctx->search);
+    if (e != cudaSuccess) { bsj_destroy(ctx); return BSJ_ERR_CUDA; }
     *out = ctx;
     return BSJ_OK;
 }
@@ -1039,7 +1236,9 @@ int64_t bsj_plan_launches(const bsj_plan* p)
     // fixed by the plan shape: per group 1 + maxN*(select? + heap?) + (maxN-1)*(gather_v1? + step
     // launches per NQ class); one finalize
     int64_t n = 1;
-    for (const auto& gr : p->groups) {
+    const bool res = uses_search(p);
+    if (res) n += (int64_t)p->search[p->select_cluster ? 0 : 1].size();
+    for (const auto& gr : res ? p->rest_groups : p->groups) {
         const int64_t per = (gr.has_gpu ? 1 : 0) + (gr.has_compat ? 1 : 0);
         const int64_t nq = __builtin_popcount((unsigned)gr.nq_mask);
         n += nq + (int64_t)gr.maxN * per + (int64_t)(gr.maxN - 1) * (nq + (gr.has_v1 ? 1 : 0));
@@ -1169,8 +1368,9 @@ bsj_status bsj_plan_autotune(bsj_plan* p, void* stream, int32_t repeats, int32_t
     cudaSetDevice(ctx->device);
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
     if (repeats < 1) repeats = 1;
-    // a uniform size that the rule already gives every group is not timed twice
-    int rule_uniform = -1;
+    // a uniform size that the rule already gives every group is not timed twice (the rule
+    // gives no k_step form to beams the resident search takes)
+    int rule_uniform = p->nrest < p->nseg ? -2 : -1;
     for (const auto& gr : p->groups) {
         if (rule_uniform == -1) rule_uniform = gr.rule_var;
         else if (rule_uniform != gr.rule_var) rule_uniform = -2;

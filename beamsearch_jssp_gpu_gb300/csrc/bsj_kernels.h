@@ -64,6 +64,59 @@ struct HeapCfg {
     int32_t kmax, chunk, ab, nmax;
 };
 
+// ---- resident search (bsj_search.cu): all levels of a gpu-mode beam in one kernel ----
+constexpr int kSearchThreads = 512;
+constexpr int kSearchBinBits = 10;
+constexpr int kSearchBins = 1 << kSearchBinBits;   // score bins of the selection
+constexpr int kSearchMaxCluster = 16;
+constexpr int kSearchNarrow = 4;       // blocks per beam at most with the cluster forms switched off
+constexpr int kSearchMinBuf = 2048;    // keys the sort's buffer holds at least
+constexpr int kSearchMinList = 1024;   // candidate keys the list holds at least
+
+// Snapshot by ready position (bytes): i32 tr[m] | i32 jr[n] | u16 op[n] | u8 mc[n] |
+// u16 r, u16 ns, i32 cmax, u32 lineage, u32 stamp (16-byte aligned).
+struct SearchLay {
+    int off_jr, off_op, off_mc, off_hdr, bytes;
+    __host__ __device__ __forceinline__ SearchLay(int n, int m)
+    {
+        off_jr = 4 * m;
+        off_op = off_jr + 4 * n;
+        off_mc = (off_op + 2 * n + 3) & ~3;
+        off_hdr = (off_mc + n + 15) & ~15;
+        bytes = off_hdr + 16;
+    }
+};
+
+// One launch: its beams, blocks per beam, lanes per survivor and shared-memory layout.
+struct SearchCfg {
+    const int32_t* list;        // the launch's beams
+    unsigned long long* spill;  // candidate keys past list_cap (offsets as StepArgs::keys)
+    int32_t cluster, lanes, rs, stage_stride, bins_per, per4_magic;
+    uint32_t c_magic;
+    int32_t list_cap, buf_cap;
+    int32_t wide;               // report the cluster route
+    int32_t off_mask, off_sel, off_info, off_list, off_stage;
+    size_t smem;
+};
+
+bool search_layout(SearchCfg& cf, int cluster, int lanes, int kmax, int nmax, int opsmax, int smax, size_t limit);
+// The current device's limits: dynamic shared memory of a block, clusters of each size that
+// run at once.
+struct SearchDevice {
+    size_t smem = 0;
+    int clusters[kSearchMaxCluster + 1] = {};
+};
+constexpr int kSearchSizes[] = {1, 2, 4, 8, 12, 16};   // blocks per beam
+cudaError_t search_device(SearchDevice& out);
+// Estimated microseconds per level with C blocks (for choosing C only).
+double search_level_us(int n, int K, bool v1, int C);
+// Blocks per beam with the smallest estimate among sizes up to cmax that the device runs and
+// whose layout fits; 0 if there is none.
+int search_blocks(const SearchDevice& dev, int n, int m, int K, bool v1, int cmax);
+// Lanes per survivor for C blocks.
+int search_lanes(int n, int K, int C);
+cudaError_t launch_search(const StepArgs& a, const SearchCfg& cf, int nbeams, bool v1, cudaStream_t stream);
+
 // Grid / shared-memory sizing helpers.
 size_t step_smem_bytes(int sb_max, int max_n, int chunk);
 size_t select_smem_bytes(int sort_cap);

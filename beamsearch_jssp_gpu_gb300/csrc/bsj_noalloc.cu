@@ -18,8 +18,8 @@
 // whose work overlaps on the GPU (different streams or threads, same device) race on the
 // array and must be serialised by the caller.
 //
-// The kernels are the library's ordinary level kernels (k_step, k_select, k_finalize);
-// only the buffers they are handed differ.  The per-call initial values reach the scratch
+// The kernels are the library's ordinary ones (the resident search, or where its buffers do
+// not fit the scratch the level kernels); only the buffers they are handed differ.  The per-call initial values reach the scratch
 // as kernel parameters, not as copies from host memory, so a call only enqueues work on
 // its stream and returns.
 #include <algorithm>
@@ -172,11 +172,30 @@ extern "C" bsj_status bsj_solve_noalloc(int32_t n, int32_t m, const int32_t* d_m
     const size_t o_pos = take(2 * align_up(K * n, 256));
     const size_t o_noise = take(1000 * sizeof(float));
     if (o > kScratchBytes) return BSJ_ERR_LIMIT;  // beam_width x n*m too large for the scratch
+    // the resident search's buffers over the same scratch, where they fit: its snapshots are
+    // larger, its overflow list is a second set of keys, and it needs no position tables
+    const SearchLay L(n, m);
+    size_t q = o_beam;
+    auto place = [&](size_t bytes) { const size_t at = q; q = align_up(q + bytes, 256); return at; };
+    const size_t s_beam = place(2 * align_up(K * L.bytes, 256));
+    const size_t s_keys = place(K * n * 8);
+    const size_t s_spill = place(K * n * 8);
+    const size_t s_sel = place(K * 4);
+    const size_t s_mask = place(K * d.words * 4);
+    const size_t s_hist = place(N * K * 4);
+    const size_t s_seq = place(N * 4);
+    const size_t s_noise = place(1000 * sizeof(float));
+    SearchDevice dev_search;
+    if (search_device(dev_search) != cudaSuccess) return BSJ_ERR_CUDA;
+    const int blocks = m >= 2 && q <= kScratchBytes
+                           ? search_blocks(dev_search, n, m, beam_width, false, kSearchMaxCluster) : 0;
     d.beam_off[0] = 0;
     d.beam_off[1] = (int64_t)align_up(K * d.sbytes, 256);
     d.key_off = d.sel_off = d.mask_off = d.hist_off = d.aux_off = d.seq_off = d.slot_off = 0;
     d.pos_off[0] = 0;
     d.pos_off[1] = (int64_t)align_up(K * n, 256);
+    const size_t beam_bytes = 2 * align_up(K * (blocks ? (size_t)L.bytes : (size_t)d.sbytes), 256);
+    if (blocks) d.beam_off[1] = (int64_t)align_up(K * L.bytes, 256);
 
     void* base_v = nullptr;
     if (scratch_address(&base_v) != cudaSuccess) return BSJ_ERR_CUDA;
@@ -221,6 +240,16 @@ extern "C" bsj_status bsj_solve_noalloc(int32_t n, int32_t m, const int32_t* d_m
     a.pos_pool = base + o_pos;
     a.noise = reinterpret_cast<const float*>(base + o_noise);
 
+    if (blocks) {
+        a.beam_pool = base + s_beam;
+        a.keys = reinterpret_cast<unsigned long long*>(base + s_keys);
+        a.sel = reinterpret_cast<uint32_t*>(base + s_sel);
+        a.masks = reinterpret_cast<uint32_t*>(base + s_mask);
+        a.hist = reinterpret_cast<uint32_t*>(base + s_hist);
+        a.seq_pool = reinterpret_cast<int32_t*>(base + s_seq);
+        a.noise = reinterpret_cast<const float*>(base + s_noise);
+    }
+
     int sort_cap = 1;
     while (sort_cap < beam_width) sort_cap <<= 1;
     int sms = 0, dev = 0;
@@ -238,19 +267,28 @@ extern "C" bsj_status bsj_solve_noalloc(int32_t n, int32_t m, const int32_t* d_m
                                     reinterpret_cast<int32_t*>(base + o_cprefix),
                                     reinterpret_cast<int32_t*>(base + o_group));
     if (cudaGetLastError() != cudaSuccess) return BSJ_ERR_CUDA;
-    if (cudaMemsetAsync(base + o_beam, 0, 2 * align_up(K * d.sbytes, 256), s) != cudaSuccess) return BSJ_ERR_CUDA;
+    if (cudaMemsetAsync(a.beam_pool, 0, beam_bytes, s) != cudaSuccess) return BSJ_ERR_CUDA;
     k_noalloc_pack<<<1, 256, 0, s>>>(d_machine, d_duration, d.N, m, reinterpret_cast<uint32_t*>(base + o_ops),
                                      reinterpret_cast<SegState*>(base + o_state));
     if (cudaGetLastError() != cudaSuccess) return BSJ_ERR_CUDA;
-    if (launch_noise_table(reinterpret_cast<float*>(base + o_noise), nullptr, s) != cudaSuccess) return BSJ_ERR_CUDA;
-    if (launch_step(a, -1, grid, nq_mask, s) != cudaSuccess) return BSJ_ERR_CUDA;
-    for (int lv = 0; lv < d.N; lv++) {
-        if (launch_select(a, lv, sort_cap, s) != cudaSuccess) return BSJ_ERR_CUDA;
-        if (lv < d.N - 1 && launch_step(a, lv, grid, nq_mask, s) != cudaSuccess) return BSJ_ERR_CUDA;
+    if (launch_noise_table(const_cast<float*>(a.noise), nullptr, s) != cudaSuccess) return BSJ_ERR_CUDA;
+    if (blocks) {
+        SearchCfg cf{};
+        search_layout(cf, blocks, search_lanes(n, beam_width, blocks), beam_width, n, d.N, L.bytes, dev_search.smem);
+        cf.list = reinterpret_cast<const int32_t*>(base + o_prefix);   // prefix[0] = 0, the one beam
+        cf.spill = reinterpret_cast<unsigned long long*>(base + s_spill);
+        cf.wide = 1;
+        if (launch_search(a, cf, 1, false, s) != cudaSuccess) return BSJ_ERR_CUDA;
+    } else {
+        if (launch_step(a, -1, grid, nq_mask, s) != cudaSuccess) return BSJ_ERR_CUDA;
+        for (int lv = 0; lv < d.N; lv++) {
+            if (launch_select(a, lv, sort_cap, s) != cudaSuccess) return BSJ_ERR_CUDA;
+            if (lv < d.N - 1 && launch_step(a, lv, grid, nq_mask, s) != cudaSuccess) return BSJ_ERR_CUDA;
+        }
     }
     if (launch_finalize(a, s) != cudaSuccess) return BSJ_ERR_CUDA;
     k_noalloc_out<<<1, 256, 0, s>>>(reinterpret_cast<const SegState*>(base + o_state),
-                                    reinterpret_cast<const int32_t*>(base + o_seq), d.N, d_out);
+                                    a.seq_pool, d.N, d_out);
     if (cudaGetLastError() != cudaSuccess) return BSJ_ERR_CUDA;
     return BSJ_OK;
 }

@@ -255,12 +255,13 @@ class Plan:
     def chunk(self, value: int):
         self.ctx._check(self.lib.bsj_plan_set_chunk(self.h, int(value)))
 
-    KERNELS = ("k_step", "k_select", "k_heap", "k_gather_v1", "k_finalize")
+    KERNELS = ("k_step", "k_select", "k_heap", "k_gather_v1", "k_finalize", "k_search")
 
     def kernel_ms(self) -> dict:
-        ms = (ctypes.c_float * 5)()
-        cnt = (ctypes.c_int64 * 5)()
-        self.ctx._check(self.lib.bsj_plan_kernel_ms(self.h, ms, cnt, 5))
+        count = len(self.KERNELS)
+        ms = (ctypes.c_float * count)()
+        cnt = (ctypes.c_int64 * count)()
+        self.ctx._check(self.lib.bsj_plan_kernel_ms(self.h, ms, cnt, count))
         return {k: (float(ms[i]), int(cnt[i])) for i, k in enumerate(self.KERNELS)}
 
 

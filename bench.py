@@ -337,8 +337,9 @@ def gpu_arm(args) -> int:
 
     # roofline of the dominant kernel (CUDA-event times of the profiled step)
     peaks = _peaks()
-    alg = {"k_step": stats["step_bytes"], "k_select": stats["select_bytes"]}
-    dom = max(("k_step", "k_select"), key=lambda k: kms[k][0])
+    alg = {"k_step": stats["step_bytes"], "k_select": stats["select_bytes"],
+           "k_search": stats["step_bytes"] + stats["select_bytes"]}
+    dom = max(alg, key=lambda k: kms[k][0])
     ms, nl = kms[dom]
     per_launch_bytes = alg[dom] / nl
     achieved = per_launch_bytes / (ms / nl / 1000.0) / 1e9
@@ -347,9 +348,9 @@ def gpu_arm(args) -> int:
                 "frac": achieved / peaks["hbm_gbs"], "traffic": traffic,
                 "algorithmic_bytes_per_launch": per_launch_bytes, "avg_launch_us": 1000.0 * ms / nl,
                 "peak_source": peaks["source"],
-                "regime": "latency-bound: each level of a beam is a dependent chain (select on a 2- or 4-SM "
-                          "cluster, then materialise+expand); the per-level set (~5 MB per beam) stays "
-                          "L2-resident, so neither HBM bandwidth nor an SM pipe is saturated",
+                "regime": "latency-bound: each level of a beam is a dependent chain (materialise + expand, "
+                          "bin, exchange, rank) on a cluster of up to 16 SMs; the per-level set (~5 MB per "
+                          "beam) stays L2-resident, so neither HBM bandwidth nor an SM pipe is saturated",
                 "kernel_share": {k: v[0] / max(1e-9, sum(x[0] for x in kms.values())) for k, v in kms.items()}}
 
     extras = {}

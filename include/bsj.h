@@ -157,7 +157,8 @@ bsj_status bsj_plan_stats(const bsj_plan *plan, double *step_bytes, double *sele
                           int64_t *expanded, int64_t *materialized, int64_t *select_fallbacks);
 /* When enabled, bsj_plan_run records CUDA events around every launch of each kernel
    class; bsj_plan_kernel_ms returns total ms per class and launch counts for the last run:
-   index 0 k_step, 1 k_select, 2 k_heap, 3 k_gather_v1, 4 k_finalize. */
+   index 0 k_step, 1 k_select, 2 k_heap, 3 k_gather_v1, 4 k_finalize, 5 k_search (the
+   resident search: all levels of a beam in one launch). */
 bsj_status bsj_plan_set_timing(bsj_plan *plan, int enable);
 bsj_status bsj_plan_kernel_ms(const bsj_plan *plan, float *ms, int64_t *launches, int count);
 
@@ -180,7 +181,12 @@ bsj_status bsj_plan_kernel_ms(const bsj_plan *plan, float *ms, int64_t *launches
    BSJ_SELECT_FORCE_CLUSTER and BSJ_SELECT_NO_CLUSTER; with any other flag set the cluster
    form runs the one-block routes on its first block.
    bsj_plan_select_routes: BSJ_ROUTE_* bits of the routes the last run took (OR over the
-   plan's beams and levels; waits for the run). */
+   plan's beams and levels; waits for the run).
+   With no flags and no forced k_step form the gpu modes run the resident search (m >= 2):
+   one launch for all levels, 1 to 16 thread blocks per beam.  It reports a level's class:
+   LARGE for more than 16384 candidate keys or K > 8192, CLUSTER for more than 4096 keys
+   split over several blocks, DIRECT otherwise; levels whose tied scores exceed its buffers
+   run the one-block routes and report those too. */
 #define BSJ_SELECT_FORCE_LARGE 1  /* large-level route (keys read in place) at any size */
 #define BSJ_SELECT_NO_LARGE    2  /* never the large-level route */
 #define BSJ_SELECT_NO_DIRECT   4  /* compact the survivors first (no direct staged pass) */
@@ -201,10 +207,10 @@ bsj_status bsj_plan_kernel_ms(const bsj_plan *plan, float *ms, int64_t *launches
 #define BSJ_ROUTE_CLUSTER  256
 bsj_status bsj_plan_set_select_route(bsj_plan *plan, int32_t flags);
 bsj_status bsj_plan_select_routes(bsj_plan *plan, uint32_t *routes);
-/* enable = 0: one thread block per beam for this plan's selections from its next run on,
-   whatever K (a throughput choice: the cluster form spends about twice the SM time per
-   level for its lower latency); enable != 0 (the default): the cluster form where the
-   rule picks it.  Both forms' graphs are kept, so switching costs one capture per form;
+/* enable = 0: the narrow forms for this plan from its next run on, whatever K (a throughput
+   choice: the cluster forms spend more SM time per level for their lower latency) -- the
+   resident search with at most 4 thread blocks per beam, and one block per beam for the
+   level kernels' selections; enable != 0 (the default): as wide as the rule picks.  Both forms' graphs are kept, so switching costs one capture per form;
    the results never depend on it.  The route flags above take precedence. */
 bsj_status bsj_plan_set_select_cluster(bsj_plan *plan, int32_t enable);
 
