@@ -1378,20 +1378,20 @@ __global__ void __launch_bounds__(kSelectThreads) k_select_cl(StepArgs a, int s,
 // 22-39, cpu/v1_pms/solver.cpp:26-62, insert_into_beam jssp_types.h:47-58).
 //
 // The survivors and their order (the next level's parent order) are what libstdc++'s
-// bounded heap holds after every child has been offered in generation order, so the heap
-// stays serial: lane 0 of warp 0 runs it and nothing else.  Warps 1..7 work one chunk of
-// parents ahead of it:
+// bounded heap holds after every child has been offered in generation order, so its
+// operations stay in order: warp 0 runs them (PipedHeap) and nothing else.  Warps 1..7 work
+// one chunk of parents ahead of it:
 //   1. stage the chunk's child tables (written by k_step) in shared memory;
 //   2. consume the glibc rand() stream.  ICH draws one value per child, so the chunk's
 //      draws are known in advance and one warp generates them 31 at a time
 //      (warp_rand_fill).  BS-PMS draws a pivot and then one value per child on the pivot's
-//      machine, so one lane walks the parents, reading each position's machine count from
-//      a table the warps built with a histogram per parent;
+//      machine, so one warp generates the stream ahead and walks the parents, reading each
+//      position's machine count from a table the warps built with a histogram per parent;
 //   3. score every child (thread per child) and drop those the heap would reject anyway:
 //      once the heap is full its front only decreases, so a key that is not below a front
 //      published earlier is not below the front when its turn comes;
-//   4. compact the remaining children, in generation order, into the buffer the heap
-//      thread reads on its next pass.
+//   4. compact the remaining children, in generation order, into the buffer the heap's
+//      warp reads on its next pass.
 // ------------------------------------------------------------------------------------
 constexpr int kHeapProducers = kHeapThreads - 32;
 constexpr int kHeapProducerWarps = kHeapProducers / 32;
@@ -1399,7 +1399,7 @@ constexpr int kHeapMiscBytes = 128 + kHeapProducerWarps * 64 * 4;
 
 __host__ __device__ __forceinline__ size_t hl_align(size_t x) { return (x + 15) & ~(size_t)15; }
 
-// hk [K] u64 | hv [K] u32 | misc | per-parent coff [C+1], pm [C], rbase [C] | rb [34 + C(n+1)]
+// hk [K + 2] u64 | hv [K + 2] u32 (node i at i + 1: two children share a 16-byte word) | misc | per-parent coff [C+1], pm [C], rbase [C] | rb [34 + C(n+1)]
 // u32 | stage [C] child tables | cpar, cpos [C n] u8 | cdraw [C n] u32 | cntv [C n] u8 |
 // ck [2][C n] u64 | cv [2][C n] u32
 struct HeapLayout {
@@ -1409,15 +1409,15 @@ struct HeapLayout {
         const size_t C = (size_t)c.chunk, cap = (size_t)c.chunk * (size_t)c.nmax;
         size_t o = 0;
         hk = o;
-        o += 8 * (size_t)c.kmax;
+        o = hl_align(o + 8 * ((size_t)c.kmax + 2));
         hv = o;
-        o = hl_align(o + 4 * (size_t)c.kmax);
+        o = hl_align(o + 4 * ((size_t)c.kmax + 2));
         misc = o;
         o += kHeapMiscBytes;
         pp = o;
         o = hl_align(o + 4 * (3 * C + 1));
         rb = o;
-        o = hl_align(o + 4 * (34 + C * ((size_t)c.nmax + 1)));
+        o = hl_align(o + 4 * (34 + C * ((size_t)c.nmax + 1) + 2 * 124));
         stage = o;
         o = hl_align(o + C * (size_t)c.ab);
         cpar = o;
@@ -1447,53 +1447,196 @@ int heap_pick_chunk(HeapCfg c, size_t budget)
     return 0;
 }
 
-// libstdc++ __push_heap: the value rises from `hole` while its parent is smaller.  The
-// parent's value is loaded with its key, so a move costs one shared-memory round trip.
-__device__ __forceinline__ void heap_sift_up(unsigned long long* hk, uint32_t* hv, int hole, int top,
-                                             unsigned long long vk, uint32_t vv)
+// libstdc++ push_heap onto `size` elements, by one warp: lane d holds the ancestor of depth d
+// of the new position; x goes below the last that is not smaller, the others move down.
+__device__ __forceinline__ void heap_push(unsigned long long* hk, uint32_t* hv, int size, unsigned long long xk,
+                                          uint32_t xv, int lane)
 {
-    while (hole > top) {
-        const int parent = (hole - 1) / 2;
-        const unsigned long long kp = hk[parent];
-        const uint32_t vp = hv[parent];
-        if (!(kp < vk)) break;
-        hk[hole] = kp;
-        hv[hole] = vp;
-        hole = parent;
+    const int D = 31 - __clz(size + 1);
+    const int pos = lane <= D ? (size + 1) >> (D - lane) : 0;   // at [pos], node pos - 1
+    const unsigned long long k = lane < D ? hk[pos] : 0ull;
+    const uint32_t v = lane < D ? hv[pos] : 0u;
+    const unsigned lt = __ballot_sync(FULL_MASK, lane < D && k < xk);
+    const int at = lt ? __ffs(lt) - 1 : D;
+    const unsigned long long uk = __shfl_up_sync(FULL_MASK, k, 1);
+    const uint32_t uv = __shfl_up_sync(FULL_MASK, v, 1);
+    if (lane >= at && lane <= D) {
+        hk[pos] = lane == at ? xk : uk;
+        hv[pos] = lane == at ? xv : uv;
     }
-    hk[hole] = vk;
-    hv[hole] = vv;
+    __syncwarp();
 }
 
-// libstdc++ __adjust_heap: the hole walks down to a leaf along the larger children (the
-// right one on ties, a lone left child is taken), then the value is pushed up from there.
-// Both children's keys and values are loaded together, so each level of the walk costs
-// one shared-memory round trip (the value no longer waits for the comparison).  (Loading
-// the four grandchildren as well, two levels per round, measured slower: 4.94 vs 4.64 s
-// per 8-beam BS-PMS search at 50x20, K=4096 -- the heap thread is issue-bound by then.)
-__device__ void heap_adjust(unsigned long long* hk, uint32_t* hv, int hole, int len,
-                            unsigned long long vk, uint32_t vv)
-{
-    const int top = hole;
-    int child = hole;
-    while (child < (len - 1) / 2) {
-        child = 2 * (child + 1);
-        const unsigned long long kr = hk[child], kl = hk[child - 1];
-        const uint32_t vr = hv[child], vl = hv[child - 1];
-        const bool left = kr < kl;
-        child -= left ? 1 : 0;
-        hk[hole] = left ? kl : kr;
-        hv[hole] = left ? vl : vr;
-        hole = child;
+// The full heap of one beam, in one warp, with replace operations (pop_heap, overwrite the
+// back, push_heap) overlapping.  libstdc++'s steps leave exactly this:
+//   pop_heap: the last element v fills the hole that starts at the root and walks to the larger
+//     child (the right one on ties) while that child is not below v.  (__adjust_heap walks to
+//     the leaf and pushes v up again; keys on the path do not increase, so v ends in the same
+//     place.)
+//   push_heap: the new element x goes into the fixed path from the last position to the root,
+//     below its last key that is not smaller; what was there moves down one.
+// Lane d < 16 holds the path's node of depth d (f) and its sibling (s) in registers.  One
+// ballot finds the depth e at which the hole leaves the path; everything on the path is then
+// two shuffled shifts.  What is left of the walk -- v sinking below s(e) -- touches only s(e)'s
+// subtree, and the next operation needs only s(e)'s new key, the walk's first step.  So the
+// walk becomes a task of a lane >= 16 that sinks two levels per later operation while those
+// run; a walk behind it in the same subtree stays two levels above and never reads its hole.
+//
+// Bound by one warp's chain of dependent instructions: ~750 cycles per replace whatever K
+// (1 300 at K=1 024 for one thread walking the whole path, growing with log K), ~160 per push
+// (325).  GB300, ms per call: 10x5 K=64 BS-ICH 4.88 -> 2.82; 8 BS-PMS beams of 30x20 K=1 024
+// 491 -> 262.  Checked on the CPU against libstdc++ over 192 000 tie-heavy replaces.
+struct PipedHeap {
+    struct Kids { ulonglong2 k; uint2 v; };
+    unsigned long long* hk;   // node i at hk[i + 1], hv[i + 1]
+    uint32_t* hv;
+    int K, D;                 // size; depth of the last position
+    int fpos, spos;           // lane d: positions of f and s
+    bool has_s, s_right;      // lane d: s exists in [0, K - 1); s is the right child
+    unsigned long long fk, sk, tk;
+    uint32_t fv, sv, tv;
+    int tpos;                 // lanes >= 16: the task's hole, -1 = none
+    Kids ka;                  // its children
+    int turn;
+
+    __device__ __forceinline__ void load(unsigned long long* k, uint32_t* v, int size, int lane)
+    {
+        hk = k;
+        hv = v;
+        K = size;
+        D = 31 - __clz(K);
+        // node d of the path to position K - 1: the leading d + 1 bits of K, less 1
+        fpos = lane <= D ? (K >> (D - lane)) - 1 : 0;
+        spos = (fpos & 1) ? fpos + 1 : fpos - 1;
+        s_right = (fpos & 1) != 0;
+        has_s = lane >= 1 && lane <= D && spos < K - 1;
+        fk = lane <= D ? hk[fpos + 1] : 0ull;
+        fv = lane <= D ? hv[fpos + 1] : 0u;
+        sk = has_s ? hk[spos + 1] : 0ull;
+        sv = has_s ? hv[spos + 1] : 0u;
+        tpos = -1;
+        turn = 0;
+        ka = kids(-1);
     }
-    if ((len & 1) == 0 && child == (len - 2) / 2) {
-        child = 2 * (child + 1);
-        hk[hole] = hk[child - 1];
-        hv[hole] = hv[child - 1];
-        hole = child - 1;
+
+    // One level of a walk: the value (vk, vv) for the hole h and where it goes, from the
+    // children's keys and values; -1 = it stays.
+    // (no hole or no children: the words of nodes -1 and 0, not used)
+    __device__ __forceinline__ Kids kids(int h) const
+    {
+        const int at = 2 * h + 1 < K - 1 && h >= 0 ? 2 * h + 2 : 0;
+        Kids c;
+        c.k = *reinterpret_cast<const ulonglong2*>(hk + at);
+        c.v = *reinterpret_cast<const uint2*>(hv + at);
+        return c;
     }
-    heap_sift_up(hk, hv, hole, top, vk, vv);
-}
+    __device__ __forceinline__ int step(int h, const Kids& c, unsigned long long vk, uint32_t vv,
+                                        unsigned long long& ok, uint32_t& ov) const
+    {
+        const int l = 2 * h + 1;
+        const bool right = l + 1 < K - 1 && !(c.k.y < c.k.x);
+        const unsigned long long kc = right ? c.k.y : c.k.x;
+        const bool down = h >= 0 && l < K - 1 && !(kc < vk);
+        ok = down ? kc : vk;
+        ov = down ? (right ? c.v.y : c.v.x) : vv;
+        return down ? l + (right ? 1 : 0) : -1;
+    }
+
+    __device__ __forceinline__ void sink(int lane)
+    {
+        unsigned long long ok;
+        uint32_t ov;
+        const int np = step(tpos, kids(tpos), tk, tv, ok, ov);
+        __syncwarp();
+        if (tpos >= 0) {
+            hk[tpos + 1] = ok;
+            hv[tpos + 1] = ov;
+        }
+        tpos = np;
+        __syncwarp();
+    }
+
+    // Everything that does not depend on the depth e is shuffled and compared beforehand, and
+    // the tasks' loads are in flight meanwhile: ~one shuffle, three ballots and two dependent
+    // loads per operation.
+    __device__ __forceinline__ void replace(unsigned long long xk, uint32_t xv, int lane)
+    {
+        const unsigned long long vk = __shfl_sync(FULL_MASK, fk, D);
+        const uint32_t vv = __shfl_sync(FULL_MASK, fv, D);
+        const unsigned long long fd = __shfl_down_sync(FULL_MASK, fk, 1), fu = __shfl_up_sync(FULL_MASK, fk, 1),
+                                 sd = __shfl_down_sync(FULL_MASK, sk, 1);
+        const uint32_t fdv = __shfl_down_sync(FULL_MASK, fv, 1), fuv = __shfl_up_sync(FULL_MASK, fv, 1),
+                       sdv = __shfl_down_sync(FULL_MASK, sv, 1);
+        // e: where the hole leaves the path; s(e) moves up and v sinks below it unless s(e) < v
+        const unsigned bal =
+            __ballot_sync(FULL_MASK, has_s && (lane == D || (s_right ? !(sk < fk) : fk < sk)));
+        const unsigned below = __ballot_sync(FULL_MASK, sk < vk);
+        {
+            unsigned long long ok;
+            uint32_t ov;
+            const int np = step(tpos, ka, tk, tv, ok, ov);
+            if (tpos >= 0) {
+                hk[tpos + 1] = ok;
+                hv[tpos + 1] = ov;
+            }
+            tpos = np;
+        }
+        __syncwarp();
+        const int e = bal ? __ffs(bal) - 1 : D;
+        const bool moves = bal != 0u && !((below >> e) & 1u);
+        const int hole = lane >= 16 ? tpos : (moves && lane == e ? spos : -1);
+        const Kids kb = kids(hole);
+        // the path without its root and v, s(e) or v inserted; x below the last key that is not
+        // smaller; (uk, uv): the same path one place down
+        unsigned long long nk = lane >= e ? fk : fd, uk = lane > e ? fu : fk;
+        uint32_t nv = lane >= e ? fv : fdv, uv = lane > e ? fuv : fv;
+        if (lane == e - 1) { nk = moves ? sd : vk; nv = moves ? sdv : vv; }
+        if (lane == e) { uk = moves ? sk : vk; uv = moves ? sv : vv; }
+        const unsigned lt = __ballot_sync(FULL_MASK, lane < D && nk < xk);
+        const int at = lt ? __ffs(lt) - 1 : D;
+        fk = lane < at ? nk : (lane == at ? xk : uk);
+        fv = lane < at ? nv : (lane == at ? xv : uv);
+        {
+            unsigned long long ok;
+            uint32_t ov;
+            const int np = step(hole, kb, lane >= 16 ? tk : vk, lane >= 16 ? tv : vv, ok, ov);
+            if (lane >= 16) {
+                if (hole >= 0) {
+                    hk[hole + 1] = ok;
+                    hv[hole + 1] = ov;
+                }
+                tpos = np;
+            } else if (hole >= 0) {
+                sk = ok;
+                sv = ov;
+            }
+            const int p = __shfl_sync(FULL_MASK, np, e);   // the rest of the new walk
+            const int slot = 16 + (turn++ & 15);
+            if (moves && lane == slot) {
+                tpos = p;
+                tk = vk;
+                tv = vv;
+            }
+        }
+        __syncwarp();
+        ka = kids(tpos);
+    }
+
+    // all tasks done, registers back to memory
+    __device__ __forceinline__ void store(int lane)
+    {
+        while (__any_sync(FULL_MASK, tpos >= 0)) sink(lane);
+        if (lane <= D) {
+            hk[fpos + 1] = fk;
+            hv[fpos + 1] = fv;
+        }
+        if (has_s) {
+            hk[spos + 1] = sk;
+            hv[spos + 1] = sv;
+        }
+        __syncwarp();
+    }
+};
 
 // glibc rand() (TYPE_3): r[t] = r[t-31] + r[t-3] mod 2^32, rand() = r[t] >> 1.
 // rb[0..34) hold r[t0-34 .. t0-1]; writes r[t0 .. t0+cnt) to rb[34 ..).  Lane j makes
@@ -1529,8 +1672,10 @@ __global__ void __launch_bounds__(kHeapThreads) k_heap(StepArgs a, int s, HeapCf
     if (d.mode < MODE_ICH || s >= d.N) return;
     SegState& st = a.st[seg];
     const HeapLayout HL(cfg);
-    unsigned long long* hk = reinterpret_cast<unsigned long long*>(smem + HL.hk);
-    uint32_t* hv = reinterpret_cast<uint32_t*>(smem + HL.hv);
+    unsigned long long* const hk1 = reinterpret_cast<unsigned long long*>(smem + HL.hk);
+    uint32_t* const hv1 = reinterpret_cast<uint32_t*>(smem + HL.hv);
+    unsigned long long* const hk = hk1 + 1;   // hk[i], hv[i]: node i
+    uint32_t* const hv = hv1 + 1;
     uint8_t* misc = smem + HL.misc;
     unsigned long long* s_front = reinterpret_cast<unsigned long long*>(misc);      // published heap front
     unsigned long long* s_best = reinterpret_cast<unsigned long long*>(misc + 8);   // (cmax << 32 | ref) min
@@ -1621,35 +1766,43 @@ __global__ void __launch_bounds__(kHeapThreads) k_heap(StepArgs a, int s, HeapCf
                 __syncwarp();
             }
             pbar();
-            if (pt == 0) {
+            if (pw == 0) {
                 // cpu/v1_pms/solver.cpp:26-53: a parent with ready ops draws its pivot, then one
-                // noise value per ready op on the pivot's machine, in ready-list order
-                int pos = 34, k = 0;
-                uint32_t r3 = rb[31], r2 = rb[32], r1 = rb[33];
+                // noise value per ready op on the pivot's machine, in ready-list order.  The
+                // warp generates the stream ahead of the walk; every lane walks it.
+                // lane p holds parent p's ready count and its reciprocal (chunks of <= 32 parents)
+                const uint32_t rcs = lane < cnt ? (uint32_t)rc_of(lane) : 0u;
+                const uint32_t inv = rcs ? 0xFFFFFFFFu / rcs : 0u;
+                int pos = 34, have = 34, k = 0;
                 for (int p = 0; p < cnt; p++) {
-                    const int rc = rc_of(p);
-                    coff[p] = k;
-                    rbase[p] = pos;
-                    if (rc == 0) {
-                        pm[p] = -1;
-                        continue;
+                    const uint32_t rc = __shfl_sync(FULL_MASK, rcs, p), mg = __shfl_sync(FULL_MASK, inv, p);
+                    while (pos + 1 + n > have) {
+                        warp_rand_fill(rb + have - 34, 124, lane);   // (past the last position: unused)
+                        have += 124;
+                        __syncwarp();
                     }
-                    uint32_t v = rb[pos - 31] + r3;
-                    rb[pos++] = v;
-                    r3 = r2; r2 = r1; r1 = v;
-                    const int piv = (int)((v >> 1) % (uint32_t)rc);
-                    pm[p] = mc_of(p)[piv];
-                    const int c = cntv[p * n + piv];
-                    rbase[p] = pos;
-                    for (int j = 0; j < c; j++) {
-                        v = rb[pos - 31] + r3;
-                        rb[pos++] = v;
-                        r3 = r2; r2 = r1; r1 = v;
+                    int piv = -1, c = 0;
+                    if (rc > 0) {
+                        const uint32_t r = rb[pos] >> 1;
+                        uint32_t x = r - __umulhi(r, mg) * rc;   // the quotient is short by 2 at most
+                        x = x >= rc ? x - rc : x;
+                        x = x >= rc ? x - rc : x;
+                        piv = (int)x;
+                        c = cntv[p * n + piv];
+                        pos++;
                     }
+                    if (lane == 0) {
+                        coff[p] = k;
+                        rbase[p] = pos;
+                        pm[p] = piv < 0 ? -1 : (int)mc_of(p)[piv];
+                    }
+                    pos += c;
                     k += c;
                 }
-                coff[cnt] = k;
-                *s_draws = pos - 34;
+                if (lane == 0) {
+                    coff[cnt] = k;
+                    *s_draws = pos - 34;
+                }
             }
             pbar();
         }
@@ -1760,42 +1913,52 @@ __global__ void __launch_bounds__(kHeapThreads) k_heap(StepArgs a, int s, HeapCf
     if (warp > 0) produce(0);
     __syncthreads();
     int size = 0;
-    unsigned long long front = ~0ull;
+    PipedHeap heap;
     for (int q = 0; q < nchunks; q++) {
         if (warp > 0) {
             produce(q + 1);
-        } else if (lane == 0) {
+        } else {
             // insert_into_beam (jssp_types.h:47-58): push while below K, else replace the
             // front (pop_heap, overwrite the back, push_heap) when strictly better
             const int nc = s_cnt[q & 1];
             const unsigned long long* ik = ck + (size_t)(q & 1) * cap;
             const uint32_t* iv = cv + (size_t)(q & 1) * cap;
-            unsigned long long nkey = nc > 0 ? ik[0] : 0ull;
-            uint32_t nval = nc > 0 ? iv[0] : 0u;
-            for (int k = 0; k < nc; k++) {
-                const unsigned long long key = nkey;
-                const uint32_t val = nval;
-                if (k + 1 < nc) {
-                    nkey = ik[k + 1];
-                    nval = iv[k + 1];
-                }
-                if (size < K) {
-                    heap_sift_up(hk, hv, size, 0, key, val);
-                    if (++size == K) {
-                        front = hk[0];
-                        *reinterpret_cast<volatile unsigned long long*>(s_front) = front;
-                    }
-                } else if (key < front) {
-                    if (size > 1) heap_adjust(hk, hv, 0, size - 1, hk[size - 1], hv[size - 1]);
-                    heap_sift_up(hk, hv, size - 1, 0, key, val);
-                    front = hk[0];
-                    *reinterpret_cast<volatile unsigned long long*>(s_front) = front;
+            int k = 0;
+            if (size < K) {
+                const int more = min(K - size, nc);
+                for (; k < more; k++) heap_push(hk1, hv1, size++, ik[k], iv[k], lane);
+                if (size == K) {
+                    heap.load(hk1, hv1, K, lane);
+                    if (lane == 0) *reinterpret_cast<volatile unsigned long long*>(s_front) = heap.fk;
                 }
             }
-            *s_size = size;
+            // 32 children at a time; those not below the front when their turn comes are passed over
+            for (; k < nc; k += 32) {
+                const unsigned long long key = k + lane < nc ? ik[k + lane] : ~0ull;
+                const uint32_t val = k + lane < nc ? iv[k + lane] : 0u;
+                const unsigned long long front = __shfl_sync(FULL_MASK, heap.fk, 0);
+                unsigned m = __ballot_sync(FULL_MASK, key < front);
+                int j = m ? __ffs(m) - 1 : 0;
+                unsigned long long xk = __shfl_sync(FULL_MASK, key, j);
+                uint32_t xv = __shfl_sync(FULL_MASK, val, j);
+                while (m) {
+                    m &= m - 1u;
+                    j = m ? __ffs(m) - 1 : 0;
+                    const unsigned long long yk = __shfl_sync(FULL_MASK, key, j);
+                    const uint32_t yv = __shfl_sync(FULL_MASK, val, j);
+                    if (__ballot_sync(FULL_MASK, lane == 0 && xk < heap.fk)) {
+                        heap.replace(xk, xv, lane);
+                        if (lane == 0) *reinterpret_cast<volatile unsigned long long*>(s_front) = heap.fk;
+                    }
+                    xk = yk;
+                    xv = yv;
+                }
+            }
+            if (lane == 0) *s_size = size;
         }
         __syncthreads();
     }
+    if (warp == 0 && size == K) heap.store(lane);
     if (nchunks == 0 && tid == 0) *s_size = 0;
     if (tid == 32) {
         st.expanded += gen;
