@@ -1202,14 +1202,27 @@ cudaError_t search_device(SearchDevice& out)
     return cudaSuccess;
 }
 
-// Fitted to single beams on GB300 (us per level, blocks per beam): 15x15 K=256 1: 8.1; 20x15
-// K=512 1: 14.7, 4: 9.5, 8: 9.0; 30x20 K=1000 1: 31, 4: 12.1, 8: 10.2, 16: 9.8; 50x20 K=4096
-// 1: 148, 4: 39, 8: 24.6, 16: 14.9; 100x20 K=4096 4: 52, 8: 31, 16: 18.8; v1 20x15 K=1024 1: 60,
-// 4: 16.6, 8: 12.6, 16: 11.2.
+// Fitted to single beams on GB300, us per level over survivors per block (v2, 20x20): one block
+// 64: 5.8, 128: 6.4, 256: 8.1, 384: 10.5, 512: 14.6, 1 024: 27.7, 2 048: 50.6; 2 blocks +1.9, 16
+// +3.8 (barriers); lists of 50 / 100 jobs cost 1.4 / 2 times as much per survivor; v1 also
+// writes the scored children (1 024: 62.4).
 double search_level_us(int n, int K, bool v1, int C)
 {
-    const double per = (K + C - 1) / C;   // survivors per block
-    return 3.3 + (C > 1 ? 4.2 + 0.15 * C : 0.0) + per * (0.012 + 0.0005 * n + (v1 ? 0.03 : 0.0));
+    const double at[] = {64, 128, 256, 384, 512}, cost[] = {0, 0.7, 2.6, 5.2, 9.3}, slots[] = {0.9, 2.0, 4.8, 7.4, 10.0};
+    const double per = (K + C - 1) / C;
+    double f = 0, w = 0.9 * per / 64;
+    if (per >= 512) {
+        f = cost[4] + (per - 512) * 0.026;
+        w = slots[4] + (per - 512) * 0.045;
+    } else {
+        for (int i = 0; i < 4; i++)
+            if (per >= at[i] && per < at[i + 1]) {
+                const double x = (per - at[i]) / (at[i + 1] - at[i]);
+                f = cost[i] + x * (cost[i + 1] - cost[i]);
+                w = slots[i] + x * (slots[i + 1] - slots[i]);
+            }
+    }
+    return (C == 1 ? 5.6 : 7.3 + 0.14 * C) + 0.008 * n + f * std::max(1.0, 0.7 + 0.013 * n) + (v1 ? w * n / 20 : 0.0);
 }
 
 int search_lanes(int n, int K, int C)
@@ -1229,10 +1242,12 @@ int search_blocks(const SearchDevice& dev, int n, int m, int K, bool v1, int cma
     const SearchLay L(n, m);
     int best = 0;
     for (int c : kSearchSizes) {
-        if ((c > cmax && best) || dev.clusters[c] < 1) continue;
+        // 12 only as the widest allowed: its odd shares leave lanes idle (v1 20x15 K=1024: 12.2 us
+        // per level, 11.2 with 16)
+        if ((c > cmax && best) || dev.clusters[c] < 1 || (c == 12 && cmax != 12)) continue;
         SearchCfg cf;
         if (!search_layout(cf, c, search_lanes(n, K, c), K, n, n * m, L.bytes, dev.smem)) continue;
-        if (!best || search_level_us(n, K, v1, c) < search_level_us(n, K, v1, best)) best = c;
+        if (!best || search_level_us(n, K, v1, c) < 0.97 * search_level_us(n, K, v1, best)) best = c;
     }
     return best;
 }
