@@ -928,7 +928,7 @@ cudaError_t enqueue_run(bsj_plan* p, cudaStream_t s, bool capturing)
             if (e != cudaSuccess) return e;
         }
     }
-    return timed(4, [&] { return launch_finalize(a, s); });
+    return timed(4, [&] { return launch_finalize(a, p->maxN, p->has_gpu ? p->sort_cap : 0, s); });
 }
 
 constexpr size_t kPlanCache = 4;
@@ -1238,8 +1238,8 @@ int64_t bsj_plan_launches(const bsj_plan* p)
 {
     if (!p) return 0;
     // fixed by the plan shape: per group 1 + maxN*(select? + heap?) + (maxN-1)*(gather_v1? + step
-    // launches per NQ class); one finalize
-    int64_t n = 1;
+    // launches per NQ class); the lineage runs (gpu modes) and the finalisation
+    int64_t n = p->has_gpu && p->maxN > 1 ? 2 : 1;
     const bool res = uses_search(p);
     if (res) n += (int64_t)p->search[p->select_cluster ? 0 : 1].size();
     for (const auto& gr : res ? p->rest_groups : p->groups) {

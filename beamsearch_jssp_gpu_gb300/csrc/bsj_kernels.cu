@@ -2015,26 +2015,68 @@ __global__ void __launch_bounds__(kHeapThreads) k_heap(StepArgs a, int s, HeapCf
 }
 
 // ------------------------------------------------------------------------------------
-// k_finalize: result makespan and the best schedule rebuilt from the level history.
+// k_lineage, k_finalize: result makespan and the best schedule rebuilt from the level history.
+//
+// The history is a chain of N dependent loads (~0.4-0.8 us each: 0.36 ms of a 15 ms search at
+// 50x20 K=4096, 1.6 ms at 100x20 with 8 beams, whose history does not fit L2).  k_lineage
+// follows every rank through each run of 32 (64) levels at once, into the beam's key region
+// (free by now); k_finalize then takes one step per run, and its threads follow the runs side
+// by side.  GB300, us per call: 50x20 K=4096 15 210 -> 14 767, 8 beams 20 912 -> 20 114, 100x20 8
+// beams 48 420 -> 46 966, 96 mixed searches 50 313 -> 48 428.
 // ------------------------------------------------------------------------------------
-__global__ void k_finalize(StepArgs a)
+constexpr int kLineageRanks = 4;     // ranks per thread: independent loads in flight
+constexpr int kLineageThreads = 256;
+
+// levels per run: its table of N / run rows of K words fits the K * n keys
+__device__ __forceinline__ int lineage_run(const SegDesc& d) { return d.m <= 32 ? 32 : 64; }
+
+__global__ void __launch_bounds__(kLineageThreads) k_lineage(StepArgs a)
 {
-    const int seg = blockIdx.x * blockDim.x + threadIdx.x;
-    if (seg >= a.nseg) return;
-    const SegDesc& d = a.segs[seg];
-    SegState& st = a.st[seg];
+    const SegDesc& d = a.segs[blockIdx.x];
+    if (d.mode > MODE_CLEAN || a.st[blockIdx.x].best == ~0ull) return;
+    const int B = lineage_run(d), t0 = (int)blockIdx.y * B, t1 = min(t0 + B, d.N - 1), K = d.K;
+    const int r0 = (int)blockIdx.z * kLineageThreads * kLineageRanks + (int)threadIdx.x;
+    if (t0 >= t1 || r0 >= K) return;
+    const uint32_t* hist = a.hist + d.hist_off;
+    uint32_t c[kLineageRanks];
+#pragma unroll
+    for (int u = 0; u < kLineageRanks; u++) c[u] = (uint32_t)(r0 + u * kLineageThreads);
+    for (int t = t1 - 1; t >= t0; t--) {
+        uint32_t e[kLineageRanks];
+#pragma unroll
+        for (int u = 0; u < kLineageRanks; u++)
+            e[u] = c[u] < (uint32_t)K ? __ldcg(hist + (int64_t)t * K + c[u]) : kMark;
+#pragma unroll
+        for (int u = 0; u < kLineageRanks; u++) c[u] = e[u] >> 8;   // kMark >> 8 is above every rank
+    }
+    uint32_t* map = reinterpret_cast<uint32_t*>(a.keys + d.key_off) + (int64_t)blockIdx.y * K;
+#pragma unroll
+    for (int u = 0; u < kLineageRanks; u++)
+        if (r0 + u * kLineageThreads < K) map[r0 + u * kLineageThreads] = c[u];
+}
+
+__global__ void __launch_bounds__(128) k_finalize(StepArgs a)
+{
+    static_assert(kMaxJobs <= 128, "a thread per job below");
+    __shared__ uint8_t s_job[kMaxOps];
+    __shared__ int s_at[kMaxOps / 32 + 1];
+    __shared__ int s_bad;
+    const int tid = threadIdx.x;
+    const SegDesc& d = a.segs[blockIdx.x];
+    SegState& st = a.st[blockIdx.x];
     int32_t* seq = a.seq_pool + d.seq_off;
-    const int N = d.N;
+    const int N = d.N, K = d.K, n = d.n;
+    const bool gpu = d.mode <= MODE_CLEAN;
     bool found = false;
     int mk = kSentinel;
     int c = 0, job = 0;
-    if (d.mode <= MODE_CLEAN) {
+    if (gpu) {
         mk = st.bound;
         if (st.best != ~0ull) {
             const int cm = (int)(st.best >> 32);
             const uint32_t slot = (uint32_t)((st.best >> 8) & 0xFFFFFFull);
             job = (int)(st.best & 0xFFull);
-            c = (int)(slot / (uint32_t)d.n);
+            c = (int)(slot / (uint32_t)n);
             found = true;
             mk = cm < mk ? cm : mk;
         }
@@ -2046,36 +2088,54 @@ __global__ void k_finalize(StepArgs a)
             job = (int)(st.best_ref & 0xFFu);
         }
     }
-    if (found && (c >= d.K || job >= d.n)) {
-        found = false;
-        atomicOr(&st.status, kStatusBadLineage);
-    }
-    if (found) {
-        seq[N - 1] = job;
-        for (int t = N - 2; t >= 0; t--) {
-            const uint32_t e = a.hist[d.hist_off + (int64_t)t * d.K + c];
-            if (e == kMark || (int)(e >> 8) >= d.K || (int)(e & 0xFFu) >= d.n) {
-                found = false;
-                atomicOr(&st.status, kStatusBadLineage);
-                break;
+    if (tid == 0) s_bad = found && (c >= K || job >= n) ? 1 : 0;
+    __syncthreads();
+    if (found && !s_bad) {
+        // runs of B levels: the rank each is entered with, then its jobs, a thread per run
+        const int B = gpu ? lineage_run(d) : N, J = (N - 1 + B - 1) / B;
+        const uint32_t* map = reinterpret_cast<const uint32_t*>(a.keys + d.key_off);
+        if (tid == 0) {
+            s_job[N - 1] = (uint8_t)job;
+            int r = c;
+            for (int j = J - 1; j >= 0; j--) {
+                s_at[j] = r;
+                if (j > 0 && r < K) r = (int)__ldcg(map + (int64_t)j * K + r);
             }
-            seq[t] = (int)(e & 0xFFu);
-            c = (int)(e >> 8);
         }
+        __syncthreads();
+        for (int j = tid; j < J; j += blockDim.x) {
+            uint32_t r = (uint32_t)s_at[j];
+            for (int t = min((j + 1) * B, N - 1) - 1; t >= j * B; t--) {
+                const uint32_t e = r < (uint32_t)K ? __ldcg(a.hist + d.hist_off + (int64_t)t * K + r) : kMark;
+                if (e == kMark || (int)(e >> 8) >= K || (int)(e & 0xFFu) >= n) {
+                    s_bad = 1;
+                    break;
+                }
+                s_job[t] = (uint8_t)(e & 0xFFu);
+                r = e >> 8;
+            }
+        }
+        __syncthreads();
+    }
+    if (found && s_bad) {
+        found = false;
+        if (tid == 0) atomicOr(&st.status, kStatusBadLineage);
     }
     if (found) {
-        int cnt[kMaxJobs];
-        for (int j = 0; j < d.n; j++) cnt[j] = 0;
-        for (int t = 0; t < N; t++) {
-            const int j = seq[t];
-            seq[t] = j * d.m + cnt[j] + 1;
-            cnt[j]++;
+        // the k-th time a job comes up is its k-th operation
+        if (tid < n) {
+            int op = tid * d.m;
+#pragma unroll 8
+            for (int t = 0; t < N; t++)
+                if (s_job[t] == tid) seq[t] = ++op;
         }
     } else {
-        for (int t = 0; t < N; t++) seq[t] = 0;
+        for (int t = tid; t < N; t += blockDim.x) seq[t] = 0;
     }
-    st.makespan = mk;
-    st.found = found ? 1 : 0;
+    if (tid == 0) {
+        st.makespan = mk;
+        st.found = found ? 1 : 0;
+    }
 }
 
 // ------------------------------------------------------------------------------------
@@ -2297,9 +2357,16 @@ cudaError_t launch_noise_table(float* noise, double* dnoise, cudaStream_t stream
     return cudaGetLastError();
 }
 
-cudaError_t launch_finalize(const StepArgs& a, cudaStream_t stream)
+cudaError_t launch_finalize(const StepArgs& a, int max_levels, int kmax_gpu, cudaStream_t stream)
 {
-    k_finalize<<<(a.nseg + 127) / 128, 128, 0, stream>>>(a);
+    if (kmax_gpu > 0 && max_levels > 1) {
+        const int ranks = kLineageThreads * kLineageRanks;
+        const dim3 grid((unsigned)a.nseg, (unsigned)((max_levels + 31) / 32), (unsigned)((kmax_gpu + ranks - 1) / ranks));
+        k_lineage<<<grid, kLineageThreads, 0, stream>>>(a);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    k_finalize<<<a.nseg, 128, 0, stream>>>(a);
     return cudaGetLastError();
 }
 

@@ -134,7 +134,8 @@ cudaError_t launch_select(const StepArgs& a, int s, int sort_cap, cudaStream_t s
 cudaError_t launch_heap(const StepArgs& a, int s, const HeapCfg& hc, cudaStream_t stream);
 // Fills noise[0..1000) with (float)k / 1e9f (once per plan; k_step copies it per CTA).
 cudaError_t launch_noise_table(float* noise, double* dnoise, cudaStream_t stream);
-cudaError_t launch_finalize(const StepArgs& a, cudaStream_t stream);
+// `max_levels`, `kmax_gpu`: largest N, and largest K of the gpu-mode beams (0: none).
+cudaError_t launch_finalize(const StepArgs& a, int max_levels, int kmax_gpu, cudaStream_t stream);
 cudaError_t configure_kernels(int sort_cap, const HeapCfg* hc, int sb_max, int max_n);
 // Raise (never lower) the dynamic shared-memory limits of k_select and k_step to what
 // a launch with `sort_cap` / `sb_max` needs.

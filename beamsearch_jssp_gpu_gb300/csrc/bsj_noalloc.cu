@@ -286,7 +286,7 @@ extern "C" bsj_status bsj_solve_noalloc(int32_t n, int32_t m, const int32_t* d_m
             if (lv < d.N - 1 && launch_step(a, lv, grid, nq_mask, s) != cudaSuccess) return BSJ_ERR_CUDA;
         }
     }
-    if (launch_finalize(a, s) != cudaSuccess) return BSJ_ERR_CUDA;
+    if (launch_finalize(a, d.N, beam_width, s) != cudaSuccess) return BSJ_ERR_CUDA;
     k_noalloc_out<<<1, 256, 0, s>>>(reinterpret_cast<const SegState*>(base + o_state),
                                     a.seq_pool, d.N, d_out);
     if (cudaGetLastError() != cudaSuccess) return BSJ_ERR_CUDA;

@@ -36,7 +36,7 @@ def _check(ctx, mc, du, mode, K, seed, bk=500000):
             for k in ("makespan", "found", "expanded", "slots", "levels"):
                 assert got[k] == want[k], (k, what)
             assert np.array_equal(got["seq"], want["seq"]), what
-        assert plan.launches == 2, what   # the search and the finalisation
+        assert plan.launches == 3, what   # the search, the lineage runs and the finalisation
     finally:
         plan.close()
 
