@@ -66,7 +66,7 @@ struct HeapCfg {
 
 // ---- resident search (bsj_search.cu): all levels of a gpu-mode beam in one kernel ----
 constexpr int kSearchThreads = 512;
-constexpr int kSearchBinBits = 10;
+constexpr int kSearchBinBits = 9;
 constexpr int kSearchBins = 1 << kSearchBinBits;   // score bins of the selection
 constexpr int kSearchMaxCluster = 16;
 constexpr int kSearchNarrow = 4;       // blocks per beam at most with the cluster forms switched off
@@ -91,7 +91,7 @@ struct SearchLay {
 struct SearchCfg {
     const int32_t* list;        // the launch's beams
     unsigned long long* spill;  // candidate keys past list_cap (offsets as StepArgs::keys)
-    int32_t cluster, lanes, rs, stage_stride, bins_per, per4_magic;
+    int32_t cluster, lanes, rs, stage_stride;
     uint32_t c_magic;
     int32_t list_cap, buf_cap;
     int32_t wide;               // report the cluster route

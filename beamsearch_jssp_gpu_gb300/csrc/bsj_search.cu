@@ -6,18 +6,17 @@
 // block for narrow beams) keeps a beam for the whole search: block r owns the ranks
 // [r*Pc, (r+1)*Pc) of every level, its candidate keys stay in its shared memory until the
 // survivors among them are handed to the block that owns their position, and the blocks
-// meet at three cluster barriers per level:
+// meet at two cluster barriers per level:
 //
 //   step    a group of G lanes per survivor: the parent's snapshot (L2) into shared memory by
 //           one bulk copy, the selected operation applied, the child stored by one bulk copy,
 //           its candidates found (a byte compare of the ready positions' machines against the
 //           pivot machine), then a thread per candidate scores it; keys go to the block's list
-//           in slot order and are counted into 1 024 score bins
-//   #1      block r sums its share of the bins over the blocks and returns to each of them
-//           its offset in the bin and the bin's total
-//   #2      -> V, the bin T that holds rank R, each bin's first position; the keys of bins
-//           <= T go to the block(s) owning their bin's positions, in any order
-//   #3      keys are unique (score, slot) pairs, so a key's position is its bin's first
+//           and are counted into 512 score bins
+//   #1      every block reads the others' counts -> V, the bin T that holds rank R, each bin's
+//           first position; the keys of bins <= T go to the block(s) owning their bin's
+//           positions, in any order
+//   #2      keys are unique (score, slot) pairs, so a key's position is its bin's first
 //           position plus the smaller keys of the bin: counted directly in small bins, by a
 //           bitonic sort of the block's keys when a bin is large
 //
@@ -55,7 +54,7 @@ namespace {
 constexpr int T = kSearchThreads;
 constexpr int NB = kSearchBins;
 static_assert(T == kSelectThreads, "the fallback's block routines assume their block size");
-static_assert(NB == 2 * T, "two bins per thread in the bin scan");
+static_assert(NB == T, "one bin per thread in the bin scan");
 
 // ops in shared memory: (duration << 8) | last-operation-of-its-job flag | machine
 constexpr uint32_t kLastOp = 0x80u;
@@ -70,12 +69,6 @@ __device__ __forceinline__ void st_peer64(const void* p, unsigned rank, unsigned
     asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(peer_addr(p, rank)), "l"(v) : "memory");
 }
 
-__device__ __forceinline__ void st_peer128(const void* p, unsigned rank, uint4 v)
-{
-    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(peer_addr(p, rank)), "r"(v.x), "r"(v.y),
-                 "r"(v.z), "r"(v.w)
-                 : "memory");
-}
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // ---- bulk copies of snapshots (global <-> shared memory), completing on a warp's mbarrier
@@ -136,8 +129,16 @@ __device__ __forceinline__ int warp_inclusive(int x, int lane)
     return x;
 }
 
-// Exclusive prefix of v over the block and its total; ws: 32 words the caller does not
+// Exclusive prefix of v over the block, and its total; ws: 32 words the caller does not
 // reuse before the next block barrier.  One block barrier.
+__device__ __forceinline__ int block_exclusive(int v, int* ws, int lane, int warp)
+{
+    const int x = warp_inclusive(v, lane);
+    if (lane == 31) ws[warp] = x;
+    __syncthreads();
+    const int w = lane < warp ? ws[lane] : 0;
+    return __reduce_add_sync(FULL_MASK, w) + x - v;
+}
 __device__ __forceinline__ int block_exclusive(int v, int* ws, int lane, int warp, int& total)
 {
     const int x = warp_inclusive(v, lane);
@@ -195,11 +196,14 @@ struct BeamConst {
 };
 
 // Fixed part of the dynamic shared memory (bytes); the rest of the layout is SearchCfg's.
+constexpr int kRow = NB / 2 + 4;                  // words: 16-bit counts of two bins, then the valid children
 constexpr int kOffHist = 0;                       // u32[NB] this block's keys per bin
-constexpr int kOffLt = kOffHist + 4 * NB;         // u32[NB][2] keys in lower blocks, total
-constexpr int kOffBase = kOffLt + 8 * NB;         // u32[NB] first position
-constexpr int kOffCur = kOffBase + 4 * NB;        // u32[NB + 64] next position
-constexpr int kOffOwn = kOffCur + 4 * (NB + 64);  // u16[NB] first | last owning block << 8
+constexpr int kOffPack = kOffHist + 4 * NB;       // u32[kRow] the same for the other blocks
+constexpr int kOffRows = kOffPack + 4 * kRow;     // u32[blocks][kRow] every block's
+constexpr int kOffTot = kOffRows + 4 * kRow * kSearchMaxCluster;   // u32[NB] keys of all blocks
+constexpr int kOffBase = kOffTot + 4 * NB;        // u32[NB] first position
+constexpr int kOffCur = kOffBase + 4 * NB;        // u32[NB] next position
+constexpr int kOffOwn = kOffCur + 4 * NB;         // u16[NB] first | last owning block << 8
 constexpr int kOffNoise = kOffOwn + 2 * NB;       // f32[1000]
 constexpr int kOffMagic = kOffNoise + 4000;       // u32[kMaxJobs + 1] floor((2^32 - 1) / r)
 constexpr int kSubBins = 128;                     // bins of a block's window refined by exact score
@@ -242,7 +246,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
     using Mask = typename std::conditional<G == 1, unsigned long long, uint32_t>::type;
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ BeamConst B;
-    __shared__ uint4 s_pub[2];                 // valid children, min, max score bits
+    __shared__ uint4 s_pub[1];                 // min, max score bits (y, z)
     __shared__ __align__(8) unsigned long long s_bar[T / 32];
     __shared__ int s_ws[2][32];
     __shared__ int s_T, s_first, s_maxbin, s_x0, s_x1, s_mymax, s_valid, s_lcount, s_tie;
@@ -253,7 +257,9 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
     const int seg = __ldg(cf.list + blockIdx.x / (unsigned)C);
 
     uint32_t* const hist = reinterpret_cast<uint32_t*>(smem + kOffHist);
-    uint2* const lt = reinterpret_cast<uint2*>(smem + kOffLt);
+    uint32_t* const packed = reinterpret_cast<uint32_t*>(smem + kOffPack);
+    uint32_t* const rows = reinterpret_cast<uint32_t*>(smem + kOffRows);
+    uint32_t* const total = reinterpret_cast<uint32_t*>(smem + kOffTot);
     uint32_t* const binbase = reinterpret_cast<uint32_t*>(smem + kOffBase);
     uint32_t* const cur = reinterpret_cast<uint32_t*>(smem + kOffCur);
     uint16_t* const own = reinterpret_cast<uint16_t*>(smem + kOffOwn);
@@ -650,7 +656,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             __syncwarp();
         }
         if (lane == 0 && nvalid) atomicAdd(&s_valid, nvalid);
-        if (!V1) bulk_wait_read();   // the staging area is the key buffer from barrier #2 on
+        if (!V1) bulk_wait_read();   // the staging area is the key buffer from barrier #1 on
         if (tid == 0) {
             s_T = 0;
             s_first = NB;
@@ -661,62 +667,57 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
         }
 
         // ---- selection: V, threshold bin, positions
-        int V, keff, R, Pn, w0, w1, H, Tb;
+        int V, Vb, keff, R, Pn, w0, w1, H, Tb;   // Vb: valid children of lower blocks
         bool exact = false;
         int lcount;
         for (;;) {
-            csync();   // #1
+            __syncthreads();
             lcount = s_lcount;
-            uint4 v;   // {lower, total} of bins 2 tid, 2 tid + 1
+            uint32_t lower = 0, tot = 0;   // of bin tid
             if (C > 1) {
-                const int per = cf.bins_per, per4 = per >> 2;   // bins per block, a multiple of 4
-#pragma unroll 1
-                for (int x = tid; x < C * per4; x += T) {
-                    const int p = (x * cf.per4_magic) >> 20, j = (x - p * per4) * 4, bin = (int)rank * per + j;
-                    uint4 w = make_uint4(0u, 0u, 0u, 0u);
-                    if (bin < NB) w = ld_peer4(&hist[bin], p);
-                    *reinterpret_cast<uint4*>(&cur[p * per + j]) = w;
+                // counts above 16 bits saturate; such a bin never fits the buffers, and V is exact
+                if (tid < NB / 2) {
+                    const uint2 c = reinterpret_cast<const uint2*>(hist)[tid];
+                    reinterpret_cast<uint2*>(hist)[tid] = make_uint2(0u, 0u);
+                    packed[tid] = min(c.x, 0xFFFFu) | (min(c.y, 0xFFFFu) << 16);
+                } else if (tid == NB / 2) {
+                    packed[NB / 2] = (uint32_t)s_valid;
+                }
+                csync();   // #1
+                for (int x = tid; x < C * (kRow / 4); x += T) {
+                    const int p = (x * (65536 / (kRow / 4) + 1)) >> 16, j = 4 * (x - p * (kRow / 4));
+                    *reinterpret_cast<uint4*>(&rows[p * kRow + j]) = ld_peer4(&packed[j], p);
                 }
                 __syncthreads();
-#pragma unroll 1
-                for (int x = tid; x < C * per4; x += T) {
-                    const int p = (x * cf.per4_magic) >> 20, j = (x - p * per4) * 4, bin = (int)rank * per + j;
-                    uint4 lower = make_uint4(0u, 0u, 0u, 0u), total = lower;
+                const uint32_t* col = rows + (tid >> 1);
+                const int half = 16 * (tid & 1);
 #pragma unroll 4
-                    for (int q = 0; q < C; q++) {
-                        const uint4 w = *reinterpret_cast<const uint4*>(&cur[q * per + j]);
-                        if (q == p) lower = total;
-                        total.x += w.x;
-                        total.y += w.y;
-                        total.z += w.z;
-                        total.w += w.w;
-                    }
-                    if (bin < NB) {
-                        st_peer128(&lt[bin], p, make_uint4(lower.x, total.x, lower.y, total.y));
-                        st_peer128(&lt[bin + 2], p, make_uint4(lower.z, total.z, lower.w, total.w));
-                    }
+                for (int q = 0; q < C; q++) {
+                    if (q == (int)rank) lower = tot;
+                    tot += (col[q * kRow] >> half) & 0xFFFFu;
                 }
-                csync();   // #2
-                v = reinterpret_cast<const uint4*>(lt)[tid];
+                const uint32_t pv = lane < C ? rows[lane * kRow + NB / 2] : 0u;
+                V = (int)__reduce_add_sync(FULL_MASK, pv);
+                Vb = (int)__reduce_add_sync(FULL_MASK, lane < (int)rank ? pv : 0u);
             } else {
-                const uint2 hv = reinterpret_cast<const uint2*>(hist)[tid];
-                v = make_uint4(0u, hv.x, 0u, hv.y);
-                reinterpret_cast<uint4*>(lt)[tid] = v;
+                tot = hist[tid];
+                hist[tid] = 0u;
+                V = s_valid;
+                Vb = 0;
             }
-            reinterpret_cast<uint2*>(hist)[tid] = make_uint2(0u, 0u);
-            const int t0 = (int)v.y, t1 = (int)v.w;
-            const int b0 = block_exclusive(t0 + t1, s_ws[0], lane, warp, V), b1 = b0 + t0;
+            const int t0 = (int)tot, b0 = block_exclusive(t0, s_ws[0], lane, warp);
             keff = usemask ? min(P * n, B.K) : min(V, B.K);
             R = min(V, keff);
             Pn = (int)(((unsigned long long)(uint32_t)(keff + C - 1) * cf.c_magic) >> 20);
             w0 = (int)rank * Pn;
             w1 = min(w0 + Pn, R);   // positions [w0, w1) of the sort are this block's
             if (lastlv || R == 0) break;
-            reinterpret_cast<uint2*>(binbase)[tid] = make_uint2((uint32_t)b0, (uint32_t)b1);
-            reinterpret_cast<uint2*>(cur)[tid] = make_uint2((uint32_t)b0 + v.x, (uint32_t)b1 + v.z);
-            const bool in0 = t0 > 0 && b0 < R, in1 = t1 > 0 && b1 < R;
-            if (C > 1 && (in0 || in1)) {
-                // first and last owner of a bin's positions
+            total[tid] = tot;
+            binbase[tid] = (uint32_t)b0;
+            cur[tid] = (uint32_t)b0 + lower;
+            const bool in = t0 > 0 && b0 < R;
+            if (C > 1 && in) {
+                // first and last owner of the bin's positions
                 const float inv = 1.0f / (float)Pn;
                 auto owner = [&](int p) {
                     int q = (int)((float)p * inv);
@@ -724,25 +725,17 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                     q += (q + 1) * Pn <= p ? 1 : 0;
                     return q;
                 };
-                own[2 * tid] = (uint16_t)(owner(b0) | (owner(min(b1, R) - 1) << 8));
-                own[2 * tid + 1] = (uint16_t)(owner(b1) | (owner(min(b1 + t1, R) - 1) << 8));
+                own[tid] = (uint16_t)(owner(b0) | (owner(min(b0 + t0, R) - 1) << 8));
             }
-            const int big = max(in0 ? t0 : 0, in1 ? t1 : 0);
-            const int wbig = (int)__reduce_max_sync(FULL_MASK, (uint32_t)big);
-            const uint32_t occ = __ballot_sync(FULL_MASK, t0 > 0 || t1 > 0);
+            const int wbig = (int)__reduce_max_sync(FULL_MASK, in ? tot : 0u);
+            const uint32_t occ = __ballot_sync(FULL_MASK, t0 > 0);
             if (lane == 0 && wbig) atomicMax(&s_maxbin, wbig);
-            if (occ && lane == __ffs(occ) - 1) atomicMin(&s_first, 2 * tid + (t0 > 0 ? 0 : 1));
-            if (in0 && b1 >= R) s_T = 2 * tid;
-            if (in1 && b1 + t1 >= R) s_T = 2 * tid + 1;
-            if (in0 && b0 < w1 && b1 > w0) {
+            if (occ && lane == __ffs(occ) - 1) atomicMin(&s_first, tid);
+            if (in && b0 + t0 >= R) s_T = tid;
+            if (in && b0 < w1 && b0 + t0 > w0) {
                 atomicMin(&s_x0, b0);
-                atomicMax(&s_x1, b1);
+                atomicMax(&s_x1, b0 + t0);
                 atomicMax(&s_mymax, t0);
-            }
-            if (in1 && b1 < w1 && b1 + t1 > w0) {
-                atomicMin(&s_x0, b1);
-                atomicMax(&s_x1, b1 + t1);
-                atomicMax(&s_mymax, t1);
             }
             __syncthreads();
             H = s_maxbin;
@@ -806,16 +799,8 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             if (R > 0 && !lastlv) B.paths |= large ? kPathLarge : (cf.wide && C > 1 && V > kClusterMinKeys ? kPathCluster : kPathDirect);
         }
         if (lastlv || keff == 0) break;    // clean: every child pruned
-        if (!V1) bulk_wait();              // this level's children are in memory before barrier #3
-        const bool fits = R == 0 || Pn + 2 * H <= cf.buf_cap;
-        int Vb = 0;                        // valid children of lower blocks (fillers and fallback only)
-        if (keff > R || !fits) {
-            if (tid == 0) s_pub[1] = make_uint4((uint32_t)s_valid, 0u, 0u, 0u);
-            csync();
-            uint32_t pv = 0;
-            if (lane < (int)rank) pv = ld_peer(&s_pub[1].x, lane);
-            Vb = (int)__reduce_add_sync(FULL_MASK, pv);
-        }
+        if (!V1) bulk_wait();              // this level's children are in memory before barrier #2
+        const bool fits = R == 0 || (H < 0xFFFF && Pn + 2 * H <= cf.buf_cap);
         if (R > 0 && fits) {
             // ---- keys of bins <= T to their positions' owners; buf[p - first position + H]
 #pragma unroll 1
@@ -842,7 +827,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                     reinterpret_cast<uint4*>(sub)[u * T + tid] = make_uint4(0u, 0u, 0u, 0u);
                 if (tid == 0) s_tie = 0;
             }
-            csync();   // #3
+            csync();   // #2
             const int x0 = s_x0, x1 = s_x1;
             unsigned long long* const win = buf + (H - w0);   // by global position
             if (s_mymax <= kPlainBinMax) {
@@ -856,7 +841,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                         k = win[x];
                         const int bin = bin_of((uint32_t)(k >> 32));
                         f0 = (int)binbase[bin];
-                        const int ft = (int)lt[bin].y;
+                        const int ft = (int)total[bin];
                         const unsigned long long* y = win + f0;
 #pragma unroll 2
                         for (int z = tid & 1; z < ft; z += 2) c += y[z] < k ? 1 : 0;
@@ -1108,8 +1093,6 @@ bool search_layout(SearchCfg& cf, int cluster, int lanes, int kmax, int nmax, in
     const int words = (nmax + 31) / 32;
     cf.cluster = cluster;
     cf.lanes = lanes;
-    cf.bins_per = ((NB + cluster - 1) / cluster + 3) & ~3;
-    cf.per4_magic = (1 << 20) / (cf.bins_per / 4) + 1;                       // x / (bins_per / 4), x < 2 * NB
     cf.c_magic = ((1u << 20) + (uint32_t)cluster - 1) / (uint32_t)cluster;   // x / cluster, x < 2^15
     cf.stage_stride = smax + ((smax >> 4) & 1 ? 0 : 16);   // odd in 16-byte units: groups' words on distinct banks
     for (cf.rs = T / lanes; cf.rs >= 16; cf.rs /= 2) {
