@@ -359,7 +359,7 @@ void plan_searches(bsj_plan* p, std::vector<int32_t>& list, int32_t* d_list, uns
             const bool v1 = d.mode == BSJ_MODE_V1;
             const double us = d.N * search_level_us(d.n, d.K, v1, c);
             // a launch lays its shared memory out for its largest beam: a beam joins a class only
-            // where that costs neither of them survivors per round
+            // where that costs neither of them survivors per round or loads ahead
             auto fits = [&](const Class& x) {
                 if (x.c != c || x.lanes != lanes || x.v1 != v1) return false;
                 SearchCfg both, one, other;
@@ -367,7 +367,7 @@ void plan_searches(bsj_plan* p, std::vector<int32_t>& list, int32_t* d_list, uns
                 search_layout(other, c, lanes, x.kmax, x.nmax, x.opsmax, x.smax, dev.smem);
                 return search_layout(both, c, lanes, std::max(x.kmax, d.K), std::max(x.nmax, d.n),
                                      std::max(x.opsmax, d.N), std::max(x.smax, S), dev.smem) &&
-                       both.rs == one.rs && both.rs == other.rs;
+                       both.rs == one.rs && both.rs == other.rs && both.ahead == one.ahead && both.ahead == other.ahead;
             };
             auto it = std::find_if(classes.begin(), classes.end(), fits);
             if (it == classes.end()) {

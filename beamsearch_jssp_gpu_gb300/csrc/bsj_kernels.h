@@ -95,6 +95,7 @@ struct SearchCfg {
     uint32_t c_magic;
     int32_t list_cap, buf_cap;
     int32_t wide;               // report the cluster route
+    int32_t ahead;              // the staging area holds a block's whole share
     int32_t off_mask, off_sel, off_info, off_list, off_stage;
     size_t smem;
 };

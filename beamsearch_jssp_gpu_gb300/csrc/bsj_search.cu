@@ -177,6 +177,7 @@ __device__ __noinline__ void sort_window(unsigned long long* src, unsigned long 
     else if (count <= 8 * T) sort_window_e<8>(src, xs, count, x0, w0, w1, sel);
     else sort_window_e<16>(src, xs, count, x0, w0, w1, sel);
 }
+constexpr int kMaxAhead = 4;           // rounds whose parents are loaded at once
 constexpr int kSortMax = 16 * T;      // keys sort_window takes
 constexpr int kPlainBinMax = 48;      // bins up to this size: every key counts the bin's smaller ones
 constexpr int kTieMax = 256;          // largest group of equal scores ranked by counting
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ BeamConst B;
     __shared__ uint4 s_pub[1];                 // min, max score bits (y, z)
-    __shared__ __align__(8) unsigned long long s_bar[T / 32];
+    __shared__ __align__(8) unsigned long long s_bar[kMaxAhead * T / 32];   // per round and warp
     __shared__ int s_ws[2][32];
     __shared__ int s_T, s_first, s_maxbin, s_x0, s_x1, s_mymax, s_valid, s_lcount, s_tie;
 
@@ -316,7 +317,8 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
         s_lcount = 0;
     }
     load_tables();
-    if (lane == 0) bar_init(&s_bar[warp]);
+    if (lane == 0)
+        for (int k = 0; k < kMaxAhead; k++) bar_init(&s_bar[k * (T / 32) + warp]);
     __syncthreads();
     const int n = B.n, S = B.S, SP = cf.stage_stride;
     const bool usemask = B.mode != MODE_CLEAN;
@@ -333,8 +335,6 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
 
     const int sv = tid / G, gl = lane % G;
     const int gsh = (lane / G) * G;
-    uint8_t* const sb = stage + sv * SP;
-    int32_t* const tr = reinterpret_cast<int32_t*>(sb);
 
     for (int t = 0;; t++) {
         const uint32_t seed_t = B.seed + (uint32_t)t;
@@ -380,12 +380,31 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
 
         // ---- step
         int nvalid = 0;
+        // where the staging area holds the block's whole share, every round's parents are on
+        // their way before the first round starts
+        const bool ahead = !V1 && t > 0 && rounds > 1 && cf.ahead;
+        if (ahead) {
+            for (int rd = 0; rd < rounds; rd++) {
+                const int rl = rd * cf.rs + sv;
+                const bool head = gl == 0 && sv < cf.rs && rl < cnt;
+                const uint32_t heads = __ballot_sync(FULL_MASK, head);
+                unsigned long long* bar = &s_bar[rd * (T / 32) + warp];
+                if (lane == 0 && heads) bar_expect(bar, __popc(heads) * S);
+                __syncwarp();
+                if (head) {
+                    proxy_fence();
+                    bulk_load(stage + rl * SP, (t & 1 ? B.beam0 : B.beam1) + (int)((sel[rl] & ~kFillerFlag) >> 7) * S, S, bar);
+                }
+            }
+        }
 #pragma unroll 1
         for (int rd = 0; rd < rounds; rd++) {
             const int rl = rd * cf.rs + sv;
             const int r = lo + rl;
             bool act = sv < cf.rs && rl < cnt;
             uint32_t e = 0;
+            uint8_t* const sb = stage + (!V1 && cf.ahead ? rl : sv) * SP;
+            int32_t* const tr = reinterpret_cast<int32_t*>(sb);
             int32_t* const jr = reinterpret_cast<int32_t*>(sb + B.off_jr);
             uint16_t* const op = reinterpret_cast<uint16_t*>(sb + B.off_op);
             uint8_t* const mcb = sb + B.off_mc;
@@ -407,17 +426,21 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                 } else {
                     const uint32_t heads = __ballot_sync(FULL_MASK, act && gl == 0);
                     if (heads) {
-                        if (lane == 0) bar_expect(&s_bar[warp], __popc(heads) * S);
-                        __syncwarp();
-                        if (act && gl == 0) {
-                            const uint8_t* src = (t & 1 ? B.beam0 : B.beam1) + (int)((e & ~kFillerFlag) >> 7) * S;
-                            if (rd > 0) bulk_wait_read();   // this slot's child of the last round
-                            // the staging slot was last accessed through the generic proxy
-                            proxy_fence();
-                            bulk_load(sb, src, S, &s_bar[warp]);
+                        const int k = ahead ? rd : 0;
+                        unsigned long long* bar = &s_bar[k * (T / 32) + warp];
+                        if (!ahead) {
+                            if (lane == 0) bar_expect(bar, __popc(heads) * S);
+                            __syncwarp();
+                            if (act && gl == 0) {
+                                const uint8_t* src = (t & 1 ? B.beam0 : B.beam1) + (int)((e & ~kFillerFlag) >> 7) * S;
+                                if (rd > 0) bulk_wait_read();   // this slot's child of the last round
+                                // the staging slot was last accessed through the generic proxy
+                                proxy_fence();
+                                bulk_load(sb, src, S, bar);
+                            }
                         }
-                        const bool ok = bar_wait(&s_bar[warp], phase);
-                        phase ^= 1u;
+                        const bool ok = bar_wait(bar, (phase >> k) & 1u);
+                        phase ^= 1u << k;
                         if (!ok) {
                             // a copy that never completed: its survivors take no further part
                             if (lane == 0) atomicOr(&a.st[seg].status, kStatusBadSelect);
@@ -571,7 +594,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                 const bool has = x0 + lane < wtot;
                 const uint32_t en = has ? (uint32_t)lget(x) : 0u;
                 const int sv2 = (int)(en >> 16), i = (int)((en >> 8) & 255u), b = (int)(en & 255u);
-                const uint8_t* sb2 = stage + sv2 * SP;
+                const uint8_t* sb2 = stage + (!V1 && cf.ahead ? rd * cf.rs + sv2 : sv2) * SP;
                 bool valid = false;
                 int fin = 0, cm = 0, opx = 0;
                 if (has) {
@@ -1112,6 +1135,10 @@ bool search_layout(SearchCfg& cf, int cluster, int lanes, int kmax, int nmax, in
         size_t roomy = kSearchMinBuf;
         while (roomy < (size_t)pc + 4096) roomy *= 2;
         if (o + roomy * 12 + std::min(want, (size_t)pc * 128) <= limit) stage = std::max(stage, roomy * 12);
+        // the whole share staged at once (2 to kMaxAhead rounds of it)
+        const size_t whole = (size_t)pc * cf.stage_stride;
+        cf.ahead = pc > cf.rs && pc <= kMaxAhead * cf.rs && o + whole + std::min(want, (size_t)pc * 64) <= limit ? 1 : 0;
+        if (cf.ahead) stage = std::max(stage, whole);
         if (o + stage + (size_t)kSearchMinList * 8 > limit) continue;
         const size_t lst = std::min(want, limit - o - stage) & ~(size_t)15;
         cf.list_cap = (int)(lst / 8);
