@@ -1060,8 +1060,11 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
         if (R > 0) {
             const uint32_t e0 = plo + ((uint32_t)s_first << shift), e1 = plo + (((uint32_t)Tb + 1u) << shift) - 1u;
             const float f0 = __uint_as_float(e0), f1 = __uint_as_float(e1);
-            const float rho = __fdividef((float)(t + 1), (float)(t + 2));
-            const float g0 = f0 * rho, g1 = f1 * rho + 0.5f * (f1 - f0);
+            // the lowest child keeps its makespan; above, half the kept range and four units of
+            // makespan more (a narrow beam's range is a few units wide, and a prediction that
+            // misses it clamps all keys into one bin)
+            const float u = __fdividef(1.0f, (float)(t + 2));
+            const float g0 = f0 - f0 * u, g1 = f1 + 0.5f * (f1 - f0) + 4.0f * u;
             plo = __float_as_uint(g0);
             const uint32_t phi = __float_as_uint(g1);
             const int nbits = phi > plo ? 32 - __clz(phi - plo) : 0;
