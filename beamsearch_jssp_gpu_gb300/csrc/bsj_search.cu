@@ -179,9 +179,17 @@ __device__ __noinline__ void sort_window(unsigned long long* src, unsigned long 
 }
 constexpr int kMaxAhead = 4;           // rounds whose parents are loaded at once
 constexpr int kSortMax = 16 * T;      // keys sort_window takes
-constexpr int kPlainBinMax = 48;      // bins up to this size: every key counts the bin's smaller ones
-constexpr int kTieMax = 256;          // largest group of equal scores ranked by counting
-constexpr int kRecountBin = 384;      // a larger bin of predicted bins: count again, exact range
+// Where the lines between the ranking routes lie, us per level (20x15 v1 K=1024 | 30x20 K=1000 |
+// 37x11 clean K=1500 | 50x20 K=4096 | 20x15 K=16384):
+// bins up to kPlainBinMax keys: every key counts the bin's smaller ones.  48: 11.1 | 9.2 | 9.9;
+// 96: 10.4 | 8.8 | 9.8; 192: 10.3 | 9.0 | 10.5 (quadratic in the bin; 24 loses 4 % at 50x20).
+constexpr int kPlainBinMax = 96;
+// groups of equal scores up to kTieMax keys are ranked by counting, larger ones sorted with the
+// whole window.  256: 14.0 | 35.2 for the last two; 512: 13.9 | 35.2; 1 024: 13.9 | 34.6.
+constexpr int kTieMax = 1024;
+// a bin larger than kRecountBin: the level is counted again over its exact score range, which costs
+// a pass over the keys and two barriers.  384: 14.0 at 50x20 K=4096; 768 and 1 536: 13.5.
+constexpr int kRecountBin = 1536;
 
 // What a block keeps of its beam.  In shared memory, not registers: the level loop's live
 // state would otherwise spill, and local memory does not fit the L1 the shared memory leaves.
@@ -763,7 +771,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             __syncthreads();
             H = s_maxbin;
             Tb = s_T;
-            const bool coarse = H > kRecountBin;
+            const bool coarse = H > kRecountBin || Pn + 2 * H > cf.buf_cap;
             if (!coarse || exact || (!recount_ok && Pn + 2 * H <= cf.buf_cap)) {
                 // a recount that did not help (ties): no more of them for this beam while it lasts
                 if (exact) recount_ok = !coarse;
