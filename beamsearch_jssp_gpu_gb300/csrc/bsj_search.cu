@@ -208,8 +208,7 @@ struct BeamConst {
 constexpr int kRow = NB / 2 + 4;                  // words: 16-bit counts of two bins, then the valid children
 constexpr int kOffHist = 0;                       // u32[NB] this block's keys per bin
 constexpr int kOffPack = kOffHist + 4 * NB;       // u32[kRow] the same for the other blocks
-constexpr int kOffRows = kOffPack + 4 * kRow;     // u32[blocks][kRow] every block's
-constexpr int kOffTot = kOffRows + 4 * kRow * kSearchMaxCluster;   // u32[NB] keys of all blocks
+constexpr int kOffTot = kOffPack + 4 * kRow;      // u32[NB] keys of all blocks
 constexpr int kOffBase = kOffTot + 4 * NB;        // u32[NB] first position
 constexpr int kOffCur = kOffBase + 4 * NB;        // u32[NB] next position
 constexpr int kOffOwn = kOffCur + 4 * NB;         // u16[NB] first | last owning block << 8
@@ -220,7 +219,7 @@ constexpr int kSubs = 16;                         // scores per refined bin
 static_assert(kSubBins * kSubs <= 1 << (32 - kSlotBits), "group and slot share a word");
 constexpr int kOffSub = (kOffMagic + 4 * (kMaxJobs + 1) + 15) & ~15;   // u32[kSubBins][kSubs]
 constexpr int kOffRef = kOffSub + 4 * kSubBins * kSubs;                // u32[kSubBins] a score of the bin
-constexpr int kOffFree = kOffRef + 4 * kSubBins;
+constexpr int kOffRows = (kOffRef + 4 * kSubBins + 15) & ~15;          // u32[blocks][kRow] every block's
 constexpr size_t kFallbackBytes = ((kSelectSmemBytes + 15) & ~(size_t)15) + 4 * (kMaxChunks + 1);
 
 // h % r for 1 <= r <= kMaxJobs
@@ -274,7 +273,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
     uint16_t* const own = reinterpret_cast<uint16_t*>(smem + kOffOwn);
     float* const noise = reinterpret_cast<float*>(smem + kOffNoise);
     uint32_t* const magic = reinterpret_cast<uint32_t*>(smem + kOffMagic);
-    uint32_t* const ops = reinterpret_cast<uint32_t*>(smem + kOffFree);
+    uint32_t* const ops = reinterpret_cast<uint32_t*>(smem + kOffRows + 4 * kRow * C);
     uint32_t* const masks = reinterpret_cast<uint32_t*>(smem + cf.off_mask);
     uint32_t* const sel = reinterpret_cast<uint32_t*>(smem + cf.off_sel);
     int4* const info = reinterpret_cast<int4*>(smem + cf.off_info);
@@ -1132,7 +1131,7 @@ bool search_layout(SearchCfg& cf, int cluster, int lanes, int kmax, int nmax, in
     for (cf.rs = T / lanes; cf.rs >= 16; cf.rs /= 2) {
         size_t o = 0;
         auto take = [&](size_t bytes) { const size_t at = o; o = (o + bytes + 15) & ~(size_t)15; return (int)at; };
-        take(kOffFree);
+        take(kOffRows + 4 * (size_t)kRow * cluster);
         take(4 * (size_t)opsmax);
         cf.off_mask = take(4 * (size_t)pc * words);
         cf.off_sel = take(4 * (size_t)pc);
@@ -1146,9 +1145,10 @@ bool search_layout(SearchCfg& cf, int cluster, int lanes, int kmax, int nmax, in
         size_t roomy = kSearchMinBuf;
         while (roomy < (size_t)pc + 4096) roomy *= 2;
         if (o + roomy * 12 + std::min(want, (size_t)pc * 128) <= limit) stage = std::max(stage, roomy * 12);
-        // the whole share staged at once (2 to kMaxAhead rounds of it)
+        // the whole share staged at once (2 to kMaxAhead rounds of it) where that leaves the
+        // list 6 keys per survivor (the levels of 50x20 hold 3.7)
         const size_t whole = (size_t)pc * cf.stage_stride;
-        cf.ahead = pc > cf.rs && pc <= kMaxAhead * cf.rs && o + whole + std::min(want, (size_t)pc * 64) <= limit ? 1 : 0;
+        cf.ahead = pc > cf.rs && pc <= kMaxAhead * cf.rs && o + whole + std::min(want, (size_t)pc * 48) <= limit ? 1 : 0;
         if (cf.ahead) stage = std::max(stage, whole);
         if (o + stage + (size_t)kSearchMinList * 8 > limit) continue;
         const size_t lst = std::min(want, limit - o - stage) & ~(size_t)15;
