@@ -85,6 +85,9 @@ constexpr int kSelectClusterMinK = 4096;
 constexpr int kClusterMinKeys = 4096;
 constexpr int kSelectClusterWideKN = 150000;
 
+// 1 000 * this + 999 fits 32 bits: the order keys of k_heap (bsj_kernels.cu)
+constexpr int64_t kNarrowTotal = 4294966;
+
 struct SegDesc {
     int32_t n, m, N, K;
     int32_t mode;
@@ -96,7 +99,7 @@ struct SegDesc {
     int32_t op_off;     // index of this instance in the op table
     int32_t nq;         // ceil(n / 32): 32-lane groups a warp needs for the ready list
     int32_t kcnt_off;   // index of this beam's first per-chunk key count
-    int32_t pad1;
+    int32_t narrow_keys;  // ICH/PMS: the instance's total duration is at most kNarrowTotal
     int64_t beam_off[2];  // byte offsets of the two beam buffers
     int64_t slot_off;     // byte offset of the v1 child-slot buffer
     int64_t key_off;      // u64 index: candidate keys of the current level

@@ -1393,6 +1393,16 @@ __global__ void __launch_bounds__(kSelectThreads) k_select_cl(StepArgs a, int s,
 //   4. compact the remaining children, in generation order, into the buffer the heap's
 //      warp reads on its next pass.
 // ------------------------------------------------------------------------------------
+//
+// 32-bit keys, wherever they order the children exactly as the scores do (equal keys for equal
+// scores included).  BS-ICH: cmax + 0.01 (rand() % 100) orders as 100 cmax + rand() % 100.
+// BS-PMS: cmax / (s + 1) + k / 10^6 with k < 1 000 orders as 1 000 cmax + k for s + 1 <= 1 000:
+// a larger cmax adds 1 / (s + 1) >= 0.001 and k takes away at most 0.000999, so scores of
+// different pairs lie at least 10^-6 apart, and three roundings of values below 4.3 10^6 move
+// one by less than 2 10^-9.  No makespan exceeds the instance's total duration (a schedule's
+// last finish is a chain of distinct operations without gaps), so the pair fits 32 bits where
+// the total is at most kNarrowTotal.  Later levels and longer instances use 64 bits.
+constexpr int kNarrowLevels = 1000;
 constexpr int kHeapProducers = kHeapThreads - 32;
 constexpr int kHeapProducerWarps = kHeapProducers / 32;
 constexpr int kHeapMiscBytes = 128 + kHeapProducerWarps * 64 * 4;
@@ -1447,23 +1457,59 @@ int heap_pick_chunk(HeapCfg c, size_t budget)
     return 0;
 }
 
+// A heap's nodes in shared memory, node i at i + 1 (so two children share an aligned pair).
+// 64-bit keys beside their values; 32-bit keys with their value in one word, a pair in one load.
+template <typename Key>
+struct HeapNodes;
+template <>
+struct HeapNodes<unsigned long long> {
+    unsigned long long* k;
+    uint32_t* v;
+    __device__ __forceinline__ HeapNodes(uint8_t* hk, uint8_t* hv)
+        : k(reinterpret_cast<unsigned long long*>(hk)), v(reinterpret_cast<uint32_t*>(hv)) {}
+    __device__ __forceinline__ unsigned long long key(int at) const { return k[at]; }
+    __device__ __forceinline__ uint32_t val(int at) const { return v[at]; }
+    __device__ __forceinline__ void put(int at, unsigned long long key, uint32_t val) const
+    {
+        k[at] = key;
+        v[at] = val;
+    }
+    __device__ __forceinline__ void pair(int at, unsigned long long& k0, unsigned long long& k1, uint32_t& v0,
+                                         uint32_t& v1) const
+    {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(k + at);
+        const uint2 b = *reinterpret_cast<const uint2*>(v + at);
+        k0 = a.x; k1 = a.y; v0 = b.x; v1 = b.y;
+    }
+};
+template <>
+struct HeapNodes<uint32_t> {
+    uint2* kv;
+    __device__ __forceinline__ HeapNodes(uint8_t* hk, uint8_t*) : kv(reinterpret_cast<uint2*>(hk)) {}
+    __device__ __forceinline__ uint32_t key(int at) const { return kv[at].x; }
+    __device__ __forceinline__ uint32_t val(int at) const { return kv[at].y; }
+    __device__ __forceinline__ void put(int at, uint32_t key, uint32_t val) const { kv[at] = make_uint2(key, val); }
+    __device__ __forceinline__ void pair(int at, uint32_t& k0, uint32_t& k1, uint32_t& v0, uint32_t& v1) const
+    {
+        const uint4 a = *reinterpret_cast<const uint4*>(kv + at);
+        k0 = a.x; v0 = a.y; k1 = a.z; v1 = a.w;
+    }
+};
+
 // libstdc++ push_heap onto `size` elements, by one warp: lane d holds the ancestor of depth d
 // of the new position; x goes below the last that is not smaller, the others move down.
-__device__ __forceinline__ void heap_push(unsigned long long* hk, uint32_t* hv, int size, unsigned long long xk,
-                                          uint32_t xv, int lane)
+template <typename Key>
+__device__ __forceinline__ void heap_push(const HeapNodes<Key>& h, int size, Key xk, uint32_t xv, int lane)
 {
     const int D = 31 - __clz(size + 1);
-    const int pos = lane <= D ? (size + 1) >> (D - lane) : 0;   // at [pos], node pos - 1
-    const unsigned long long k = lane < D ? hk[pos] : 0ull;
-    const uint32_t v = lane < D ? hv[pos] : 0u;
+    const int pos = lane <= D ? (size + 1) >> (D - lane) : 0;   // at pos, node pos - 1
+    const Key k = lane < D ? h.key(pos) : (Key)0;
+    const uint32_t v = lane < D ? h.val(pos) : 0u;
     const unsigned lt = __ballot_sync(FULL_MASK, lane < D && k < xk);
     const int at = lt ? __ffs(lt) - 1 : D;
-    const unsigned long long uk = __shfl_up_sync(FULL_MASK, k, 1);
+    const Key uk = __shfl_up_sync(FULL_MASK, k, 1);
     const uint32_t uv = __shfl_up_sync(FULL_MASK, v, 1);
-    if (lane >= at && lane <= D) {
-        hk[pos] = lane == at ? xk : uk;
-        hv[pos] = lane == at ? xv : uv;
-    }
+    if (lane >= at && lane <= D) h.put(pos, lane == at ? xk : uk, lane == at ? xv : uv);
     __syncwarp();
 }
 
@@ -1482,27 +1528,28 @@ __device__ __forceinline__ void heap_push(unsigned long long* hk, uint32_t* hv, 
 // walk becomes a task of a lane >= 16 that sinks two levels per later operation while those
 // run; a walk behind it in the same subtree stays two levels above and never reads its hole.
 //
-// Bound by one warp's chain of dependent instructions: ~750 cycles per replace whatever K
-// (1 300 at K=1 024 for one thread walking the whole path, growing with log K), ~160 per push
-// (325).  GB300, ms per call: 10x5 K=64 BS-ICH 4.88 -> 2.82; 8 BS-PMS beams of 30x20 K=1 024
-// 491 -> 262.  Checked on the CPU against libstdc++ over 192 000 tie-heavy replaces.
+// Bound by one warp's chain of dependent instructions, whatever K: with 64-bit keys 895 cycles
+// per replace and its loop (1 300 at K=1 024 for one thread walking the whole path, growing
+// with log K), ~160 per push (325).  GB300, ms per call, one thread -> 64-bit keys -> 32-bit
+// keys: 10x5 K=64 BS-ICH 4.88 -> 2.80 -> 2.42; 8 BS-PMS beams of 30x20 K=1 024 491 -> 267 -> 230.
+// Checked on the CPU against libstdc++ over 192 000 tie-heavy replaces.
+template <typename Key>
 struct PipedHeap {
-    struct Kids { ulonglong2 k; uint2 v; };
-    unsigned long long* hk;   // node i at hk[i + 1], hv[i + 1]
-    uint32_t* hv;
+    struct Kids { Key k0, k1; uint32_t v0, v1; };
+    HeapNodes<Key> h;
     int K, D;                 // size; depth of the last position
     int fpos, spos;           // lane d: positions of f and s
     bool has_s, s_right;      // lane d: s exists in [0, K - 1); s is the right child
-    unsigned long long fk, sk, tk;
+    Key fk, sk, tk;
     uint32_t fv, sv, tv;
     int tpos;                 // lanes >= 16: the task's hole, -1 = none
     Kids ka;                  // its children
     int turn;
 
-    __device__ __forceinline__ void load(unsigned long long* k, uint32_t* v, int size, int lane)
+    __device__ __forceinline__ explicit PipedHeap(const HeapNodes<Key>& nodes) : h(nodes) {}
+
+    __device__ __forceinline__ void load(int size, int lane)
     {
-        hk = k;
-        hv = v;
         K = size;
         D = 31 - __clz(K);
         // node d of the path to position K - 1: the leading d + 1 bits of K, less 1
@@ -1510,47 +1557,43 @@ struct PipedHeap {
         spos = (fpos & 1) ? fpos + 1 : fpos - 1;
         s_right = (fpos & 1) != 0;
         has_s = lane >= 1 && lane <= D && spos < K - 1;
-        fk = lane <= D ? hk[fpos + 1] : 0ull;
-        fv = lane <= D ? hv[fpos + 1] : 0u;
-        sk = has_s ? hk[spos + 1] : 0ull;
-        sv = has_s ? hv[spos + 1] : 0u;
+        fk = lane <= D ? h.key(fpos + 1) : (Key)0;
+        fv = lane <= D ? h.val(fpos + 1) : 0u;
+        sk = has_s ? h.key(spos + 1) : (Key)0;
+        sv = has_s ? h.val(spos + 1) : 0u;
         tpos = -1;
         turn = 0;
         ka = kids(-1);
     }
 
-    // One level of a walk: the value (vk, vv) for the hole h and where it goes, from the
+    // One level of a walk: the value (vk, vv) for the hole p and where it goes, from the
     // children's keys and values; -1 = it stays.
     // (no hole or no children: the words of nodes -1 and 0, not used)
-    __device__ __forceinline__ Kids kids(int h) const
+    __device__ __forceinline__ Kids kids(int p) const
     {
-        const int at = 2 * h + 1 < K - 1 && h >= 0 ? 2 * h + 2 : 0;
         Kids c;
-        c.k = *reinterpret_cast<const ulonglong2*>(hk + at);
-        c.v = *reinterpret_cast<const uint2*>(hv + at);
+        h.pair(2 * p + 1 < K - 1 && p >= 0 ? 2 * p + 2 : 0, c.k0, c.k1, c.v0, c.v1);
         return c;
     }
-    __device__ __forceinline__ int step(int h, const Kids& c, unsigned long long vk, uint32_t vv,
-                                        unsigned long long& ok, uint32_t& ov) const
+    __device__ __forceinline__ int step(int p, const Kids& c, Key vk, uint32_t vv, Key& ok, uint32_t& ov) const
     {
-        const int l = 2 * h + 1;
-        const bool right = l + 1 < K - 1 && !(c.k.y < c.k.x);
-        const unsigned long long kc = right ? c.k.y : c.k.x;
-        const bool down = h >= 0 && l < K - 1 && !(kc < vk);
+        const int l = 2 * p + 1;
+        const bool right = l + 1 < K - 1 && !(c.k1 < c.k0);
+        const Key kc = right ? c.k1 : c.k0;
+        const bool down = p >= 0 && l < K - 1 && !(kc < vk);
         ok = down ? kc : vk;
-        ov = down ? (right ? c.v.y : c.v.x) : vv;
+        ov = down ? (right ? c.v1 : c.v0) : vv;
         return down ? l + (right ? 1 : 0) : -1;
     }
 
     __device__ __forceinline__ void sink(int lane)
     {
-        unsigned long long ok;
+        Key ok;
         uint32_t ov;
         const int np = step(tpos, kids(tpos), tk, tv, ok, ov);
         __syncwarp();
         if (tpos >= 0) {
-            hk[tpos + 1] = ok;
-            hv[tpos + 1] = ov;
+            h.put(tpos + 1, ok, ov);
         }
         tpos = np;
         __syncwarp();
@@ -1559,12 +1602,12 @@ struct PipedHeap {
     // Everything that does not depend on the depth e is shuffled and compared beforehand, and
     // the tasks' loads are in flight meanwhile: ~one shuffle, three ballots and two dependent
     // loads per operation.
-    __device__ __forceinline__ void replace(unsigned long long xk, uint32_t xv, int lane)
+    __device__ __forceinline__ void replace(Key xk, uint32_t xv, int lane)
     {
-        const unsigned long long vk = __shfl_sync(FULL_MASK, fk, D);
+        const Key vk = __shfl_sync(FULL_MASK, fk, D);
         const uint32_t vv = __shfl_sync(FULL_MASK, fv, D);
-        const unsigned long long fd = __shfl_down_sync(FULL_MASK, fk, 1), fu = __shfl_up_sync(FULL_MASK, fk, 1),
-                                 sd = __shfl_down_sync(FULL_MASK, sk, 1);
+        const Key fd = __shfl_down_sync(FULL_MASK, fk, 1), fu = __shfl_up_sync(FULL_MASK, fk, 1),
+                  sd = __shfl_down_sync(FULL_MASK, sk, 1);
         const uint32_t fdv = __shfl_down_sync(FULL_MASK, fv, 1), fuv = __shfl_up_sync(FULL_MASK, fv, 1),
                        sdv = __shfl_down_sync(FULL_MASK, sv, 1);
         // e: where the hole leaves the path; s(e) moves up and v sinks below it unless s(e) < v
@@ -1572,12 +1615,11 @@ struct PipedHeap {
             __ballot_sync(FULL_MASK, has_s && (lane == D || (s_right ? !(sk < fk) : fk < sk)));
         const unsigned below = __ballot_sync(FULL_MASK, sk < vk);
         {
-            unsigned long long ok;
+            Key ok;
             uint32_t ov;
             const int np = step(tpos, ka, tk, tv, ok, ov);
             if (tpos >= 0) {
-                hk[tpos + 1] = ok;
-                hv[tpos + 1] = ov;
+                h.put(tpos + 1, ok, ov);
             }
             tpos = np;
         }
@@ -1588,7 +1630,7 @@ struct PipedHeap {
         const Kids kb = kids(hole);
         // the path without its root and v, s(e) or v inserted; x below the last key that is not
         // smaller; (uk, uv): the same path one place down
-        unsigned long long nk = lane >= e ? fk : fd, uk = lane > e ? fu : fk;
+        Key nk = lane >= e ? fk : fd, uk = lane > e ? fu : fk;
         uint32_t nv = lane >= e ? fv : fdv, uv = lane > e ? fuv : fv;
         if (lane == e - 1) { nk = moves ? sd : vk; nv = moves ? sdv : vv; }
         if (lane == e) { uk = moves ? sk : vk; uv = moves ? sv : vv; }
@@ -1597,13 +1639,12 @@ struct PipedHeap {
         fk = lane < at ? nk : (lane == at ? xk : uk);
         fv = lane < at ? nv : (lane == at ? xv : uv);
         {
-            unsigned long long ok;
+            Key ok;
             uint32_t ov;
             const int np = step(hole, kb, lane >= 16 ? tk : vk, lane >= 16 ? tv : vv, ok, ov);
             if (lane >= 16) {
                 if (hole >= 0) {
-                    hk[hole + 1] = ok;
-                    hv[hole + 1] = ov;
+                    h.put(hole + 1, ok, ov);
                 }
                 tpos = np;
             } else if (hole >= 0) {
@@ -1627,12 +1668,10 @@ struct PipedHeap {
     {
         while (__any_sync(FULL_MASK, tpos >= 0)) sink(lane);
         if (lane <= D) {
-            hk[fpos + 1] = fk;
-            hv[fpos + 1] = fv;
+            h.put(fpos + 1, fk, fv);
         }
         if (has_s) {
-            hk[spos + 1] = sk;
-            hv[spos + 1] = sv;
+            h.put(spos + 1, sk, sv);
         }
         __syncwarp();
     }
@@ -1663,19 +1702,13 @@ __device__ void warp_rand_fill(uint32_t* rb, int cnt, int lane)
     }
 }
 
-__global__ void __launch_bounds__(kHeapThreads) k_heap(StepArgs a, int s, HeapCfg cfg)
+template <typename Key>
+__device__ __forceinline__ void heap_level(const StepArgs& a, int s, const HeapCfg& cfg, const SegDesc& d, SegState& st,
+                                           uint8_t* smem)
 {
-    pdl_wait();
-    extern __shared__ __align__(16) uint8_t smem[];
-    const int seg = a.seg_lo + blockIdx.x;
-    const SegDesc& d = a.segs[seg];
-    if (d.mode < MODE_ICH || s >= d.N) return;
-    SegState& st = a.st[seg];
+    constexpr bool narrow = sizeof(Key) == 4;
     const HeapLayout HL(cfg);
-    unsigned long long* const hk1 = reinterpret_cast<unsigned long long*>(smem + HL.hk);
-    uint32_t* const hv1 = reinterpret_cast<uint32_t*>(smem + HL.hv);
-    unsigned long long* const hk = hk1 + 1;   // hk[i], hv[i]: node i
-    uint32_t* const hv = hv1 + 1;
+    const HeapNodes<Key> nodes(smem + HL.hk, smem + HL.hv);
     uint8_t* misc = smem + HL.misc;
     unsigned long long* s_front = reinterpret_cast<unsigned long long*>(misc);      // published heap front
     unsigned long long* s_best = reinterpret_cast<unsigned long long*>(misc + 8);   // (cmax << 32 | ref) min
@@ -1696,7 +1729,7 @@ __global__ void __launch_bounds__(kHeapThreads) k_heap(StepArgs a, int s, HeapCf
     uint32_t* cdraw = reinterpret_cast<uint32_t*>(smem + HL.cdraw);
     uint8_t* cntv = smem + HL.cntv;
     const size_t cap = (size_t)C * cfg.nmax;
-    unsigned long long* ck = reinterpret_cast<unsigned long long*>(smem + HL.ck);
+    Key* ck = reinterpret_cast<Key*>(smem + HL.ck);
     uint32_t* cv = reinterpret_cast<uint32_t*>(smem + HL.cv);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1842,13 +1875,13 @@ __global__ void __launch_bounds__(kHeapThreads) k_heap(StepArgs a, int s, HeapCf
         // score, drop what the heap would reject, compact in order
         const double ns = (double)(s + 1);
         unsigned long long bmin = ~0ull;
-        unsigned long long* okey = ck + (size_t)(q & 1) * cap;
+        Key* okey = ck + (size_t)(q & 1) * cap;
         uint32_t* oval = cv + (size_t)(q & 1) * cap;
         int out = 0;
         for (int t0 = 0; t0 < T; t0 += kHeapProducers) {
             const int k = t0 + pt;
             bool keep = false;
-            unsigned long long key = 0;
+            Key key = 0;
             uint32_t val = 0;
             if (k < T) {
                 const int p = cpar[k], i = cpos[k];
@@ -1858,12 +1891,16 @@ __global__ void __launch_bounds__(kHeapThreads) k_heap(StepArgs a, int s, HeapCf
                 if (ich) {
                     // score = cmax + (rand()%100)*0.01 (cpu/v0_ich/solver.cpp:35): the pair
                     // (cmax, rand()%100) orders exactly like that double
-                    key = (unsigned long long)cc * 100ull + (dr % 100u);
+                    key = (Key)cc * 100u + (dr % 100u);
                     keep = key < F;
                 } else {
                     // cpu/v1_pms/solver.cpp:52-57
-                    const double sc = __dadd_rn(__ddiv_rn((double)cc, ns), a.dnoise[dr % 1000u]);
-                    key = (unsigned long long)__double_as_longlong(sc);
+                    if (narrow) {
+                        key = (Key)cc * 1000u + (dr % 1000u);
+                    } else {
+                        const double sc = __dadd_rn(__ddiv_rn((double)cc, ns), a.dnoise[dr % 1000u]);
+                        key = (Key)__double_as_longlong(sc);
+                    }
                     keep = cc < bound && key < F;
                     if (last && cc < kSentinel) {
                         const unsigned long long bk = ((unsigned long long)(uint32_t)cc << 32) |
@@ -1913,7 +1950,7 @@ __global__ void __launch_bounds__(kHeapThreads) k_heap(StepArgs a, int s, HeapCf
     if (warp > 0) produce(0);
     __syncthreads();
     int size = 0;
-    PipedHeap heap;
+    PipedHeap<Key> heap(nodes);
     for (int q = 0; q < nchunks; q++) {
         if (warp > 0) {
             produce(q + 1);
@@ -1921,30 +1958,30 @@ __global__ void __launch_bounds__(kHeapThreads) k_heap(StepArgs a, int s, HeapCf
             // insert_into_beam (jssp_types.h:47-58): push while below K, else replace the
             // front (pop_heap, overwrite the back, push_heap) when strictly better
             const int nc = s_cnt[q & 1];
-            const unsigned long long* ik = ck + (size_t)(q & 1) * cap;
+            const Key* ik = ck + (size_t)(q & 1) * cap;
             const uint32_t* iv = cv + (size_t)(q & 1) * cap;
             int k = 0;
             if (size < K) {
                 const int more = min(K - size, nc);
-                for (; k < more; k++) heap_push(hk1, hv1, size++, ik[k], iv[k], lane);
+                for (; k < more; k++) heap_push<Key>(nodes, size++, ik[k], iv[k], lane);
                 if (size == K) {
-                    heap.load(hk1, hv1, K, lane);
+                    heap.load(K, lane);
                     if (lane == 0) *reinterpret_cast<volatile unsigned long long*>(s_front) = heap.fk;
                 }
             }
             // 32 children at a time; those not below the front when their turn comes are passed over
             for (; k < nc; k += 32) {
-                const unsigned long long key = k + lane < nc ? ik[k + lane] : ~0ull;
+                const Key key = k + lane < nc ? ik[k + lane] : ~(Key)0;
                 const uint32_t val = k + lane < nc ? iv[k + lane] : 0u;
-                const unsigned long long front = __shfl_sync(FULL_MASK, heap.fk, 0);
+                const Key front = __shfl_sync(FULL_MASK, heap.fk, 0);
                 unsigned m = __ballot_sync(FULL_MASK, key < front);
                 int j = m ? __ffs(m) - 1 : 0;
-                unsigned long long xk = __shfl_sync(FULL_MASK, key, j);
+                Key xk = __shfl_sync(FULL_MASK, key, j);
                 uint32_t xv = __shfl_sync(FULL_MASK, val, j);
                 while (m) {
                     m &= m - 1u;
                     j = m ? __ffs(m) - 1 : 0;
-                    const unsigned long long yk = __shfl_sync(FULL_MASK, key, j);
+                    const Key yk = __shfl_sync(FULL_MASK, key, j);
                     const uint32_t yv = __shfl_sync(FULL_MASK, val, j);
                     if (__ballot_sync(FULL_MASK, lane == 0 && xk < heap.fk)) {
                         heap.replace(xk, xv, lane);
@@ -1970,7 +2007,7 @@ __global__ void __launch_bounds__(kHeapThreads) k_heap(StepArgs a, int s, HeapCf
         const int fs = *s_size;
         unsigned long long bmin = ~0ull;
         for (int r = tid; r < fs; r += blockDim.x) {
-            const uint32_t e = hv[r];
+            const uint32_t e = nodes.val(r + 1);
             const uint8_t* pa = aux + (int64_t)(e >> 8) * ab;
             const int cm = reinterpret_cast<const int32_t*>(pa + 4)[e & 0xFFu];
             if (cm < kSentinel) {
@@ -1996,7 +2033,7 @@ __global__ void __launch_bounds__(kHeapThreads) k_heap(StepArgs a, int s, HeapCf
                 best_cm = (int)(b >> 32);
                 uint32_t c, i;
                 if (ich) {
-                    const uint32_t e = hv[(uint32_t)b];
+                    const uint32_t e = nodes.val((int)(uint32_t)b + 1);
                     c = e >> 8;
                     i = e & 0xFFu;
                 } else {
@@ -2011,7 +2048,19 @@ __global__ void __launch_bounds__(kHeapThreads) k_heap(StepArgs a, int s, HeapCf
     }
     if (tid < 34) st.rng[(k0 + (uint32_t)*s_dtot + (uint32_t)tid) % 34u] = rb[tid];
     uint32_t* sel = a.sel + d.sel_off;
-    for (int r = tid; r < out_size; r += blockDim.x) sel[r] = hv[r];
+    for (int r = tid; r < out_size; r += blockDim.x) sel[r] = nodes.val(r + 1);
+}
+
+__global__ void __launch_bounds__(kHeapThreads) k_heap(StepArgs a, int s, HeapCfg cfg)
+{
+    pdl_wait();
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int seg = a.seg_lo + blockIdx.x;
+    const SegDesc& d = a.segs[seg];
+    if (d.mode < MODE_ICH || s >= d.N) return;
+    SegState& st = a.st[seg];
+    if (d.narrow_keys && (d.mode == MODE_ICH || s < kNarrowLevels)) heap_level<uint32_t>(a, s, cfg, d, st, smem);
+    else heap_level<unsigned long long>(a, s, cfg, d, st, smem);
 }
 
 // ------------------------------------------------------------------------------------
