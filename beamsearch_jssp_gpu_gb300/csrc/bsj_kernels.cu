@@ -1409,7 +1409,7 @@ constexpr int kHeapMiscBytes = 128 + kHeapProducerWarps * 64 * 4;
 
 __host__ __device__ __forceinline__ size_t hl_align(size_t x) { return (x + 15) & ~(size_t)15; }
 
-// hk [K + 2] u64 | hv [K + 2] u32 (node i at i + 1: two children share a 16-byte word) | misc | per-parent coff [C+1], pm [C], rbase [C] | rb [34 + C(n+1)]
+// hk [K + 3] u64 | hv [K + 3] u32 (node i at i + 1: two children share an aligned pair) | misc | per-parent coff [C+1], pm [C], rbase [C] | rb [34 + C(n+1)]
 // u32 | stage [C] child tables | cpar, cpos [C n] u8 | cdraw [C n] u32 | cntv [C n] u8 |
 // ck [2][C n] u64 | cv [2][C n] u32
 struct HeapLayout {
@@ -1419,9 +1419,9 @@ struct HeapLayout {
         const size_t C = (size_t)c.chunk, cap = (size_t)c.chunk * (size_t)c.nmax;
         size_t o = 0;
         hk = o;
-        o = hl_align(o + 8 * ((size_t)c.kmax + 2));
+        o = hl_align(o + 8 * ((size_t)c.kmax + 3));
         hv = o;
-        o = hl_align(o + 4 * ((size_t)c.kmax + 2));
+        o = hl_align(o + 4 * ((size_t)c.kmax + 3));
         misc = o;
         o += kHeapMiscBytes;
         pp = o;
@@ -1561,29 +1561,34 @@ struct PipedHeap {
         fv = lane <= D ? h.val(fpos + 1) : 0u;
         sk = has_s ? h.key(spos + 1) : (Key)0;
         sv = has_s ? h.val(spos + 1) : 0u;
+        __syncwarp();
+        // the words around the heap that a walk's end reads, and the root's and the last node's
+        // (in registers): no key
+        if (lane < 5) h.put(lane < 2 ? lane : K + lane - 2, (Key)0, 0u);
+        __syncwarp();
+        tk = 1;
         tpos = -1;
         turn = 0;
         ka = kids(-1);
     }
 
     // One level of a walk: the value (vk, vv) for the hole p and where it goes, from the
-    // children's keys and values; -1 = it stays.
-    // (no hole or no children: the words of nodes -1 and 0, not used)
+    // children's keys and values; -1 = it stays.  Keys are at least 1, and children that do
+    // not exist (or of no hole, p = -1) read as 0: smaller than any.
     __device__ __forceinline__ Kids kids(int p) const
     {
         Kids c;
-        h.pair(2 * p + 1 < K - 1 && p >= 0 ? 2 * p + 2 : 0, c.k0, c.k1, c.v0, c.v1);
+        h.pair(min(2 * p + 2, (K + 1) & ~1), c.k0, c.k1, c.v0, c.v1);
         return c;
     }
     __device__ __forceinline__ int step(int p, const Kids& c, Key vk, uint32_t vv, Key& ok, uint32_t& ov) const
     {
-        const int l = 2 * p + 1;
-        const bool right = l + 1 < K - 1 && !(c.k1 < c.k0);
+        const bool right = !(c.k1 < c.k0);
         const Key kc = right ? c.k1 : c.k0;
-        const bool down = p >= 0 && l < K - 1 && !(kc < vk);
+        const bool down = !(kc < vk);
         ok = down ? kc : vk;
         ov = down ? (right ? c.v1 : c.v0) : vv;
-        return down ? l + (right ? 1 : 0) : -1;
+        return down ? 2 * p + (right ? 2 : 1) : -1;
     }
 
     __device__ __forceinline__ void sink(int lane)
@@ -1891,15 +1896,15 @@ __device__ __forceinline__ void heap_level(const StepArgs& a, int s, const HeapC
                 if (ich) {
                     // score = cmax + (rand()%100)*0.01 (cpu/v0_ich/solver.cpp:35): the pair
                     // (cmax, rand()%100) orders exactly like that double
-                    key = (Key)cc * 100u + (dr % 100u);
+                    key = (Key)cc * 100u + (dr % 100u) + 1u;
                     keep = key < F;
                 } else {
                     // cpu/v1_pms/solver.cpp:52-57
                     if (narrow) {
-                        key = (Key)cc * 1000u + (dr % 1000u);
+                        key = (Key)cc * 1000u + (dr % 1000u) + 1u;
                     } else {
                         const double sc = __dadd_rn(__ddiv_rn((double)cc, ns), a.dnoise[dr % 1000u]);
-                        key = (Key)__double_as_longlong(sc);
+                        key = (Key)__double_as_longlong(sc) + 1u;
                     }
                     keep = cc < bound && key < F;
                     if (last && cc < kSentinel) {
