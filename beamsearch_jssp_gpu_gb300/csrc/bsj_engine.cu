@@ -348,6 +348,16 @@ std::vector<int> search_shares(const bsj_plan* p, int cmax_form)
             if (best.empty() || t < best_us) { best = c; best_us = t; }
         }
     }
+    // the narrow form saves SM time, and wide beams of long lists spend hardly more of it on
+    // eight blocks (100x15 K=4 096, estimated: 4 x 53.9 or 8 x 27.8 us per level)
+    if (cmax_form == kSearchNarrow && dev.clusters[8] > 0)
+        for (int i = 0; i < count; i++) {
+            const SegDesc& d = p->segs[p->nrest + i];
+            const bool v1 = d.mode == BSJ_MODE_V1;
+            if (search_blocks(dev, d.n, d.m, d.K, v1, 8) == 8 &&
+                8 * search_level_us(d.n, d.K, v1, 8) <= 1.1 * best[i] * search_level_us(d.n, d.K, v1, best[i]))
+                best[i] = 8;
+        }
     return best;
 }
 

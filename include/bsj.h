@@ -209,9 +209,10 @@ bsj_status bsj_plan_set_select_route(bsj_plan *plan, int32_t flags);
 bsj_status bsj_plan_select_routes(bsj_plan *plan, uint32_t *routes);
 /* enable = 0: the narrow forms for this plan from its next run on, whatever K (a throughput
    choice: the cluster forms spend more SM time per level for their lower latency) -- the
-   resident search with at most 4 thread blocks per beam, and one block per beam for the
-   level kernels' selections; enable != 0 (the default): as wide as the rule picks.  Both forms' graphs are kept, so switching costs one capture per form;
-   the results never depend on it.  The route flags above take precedence. */
+   resident search with at most 4 thread blocks per beam (8 for wide beams of long lists,
+   where they cost hardly more SM time), and one block per beam for the level kernels'
+   selections; enable != 0 (the default): as wide as the rule picks.  Both forms' graphs are
+   kept, so switching costs one capture per form; the results never depend on it.  The route flags above take precedence. */
 bsj_status bsj_plan_set_select_cluster(bsj_plan *plan, int32_t enable);
 
 /* ---- Autotuning (no counterpart in the reference, whose launch shape is fixed:
