@@ -1531,7 +1531,7 @@ __device__ __forceinline__ void heap_push(const HeapNodes<Key>& h, int size, Key
 // Bound by one warp's chain of dependent instructions, whatever K: with 64-bit keys 895 cycles
 // per replace and its loop (1 300 at K=1 024 for one thread walking the whole path, growing
 // with log K), ~160 per push (325).  GB300, ms per call, one thread -> 64-bit keys -> 32-bit
-// keys: 10x5 K=64 BS-ICH 4.88 -> 2.80 -> 2.42; 8 BS-PMS beams of 30x20 K=1 024 491 -> 267 -> 230.
+// keys: 10x5 K=64 BS-ICH 4.88 -> 2.80 -> 2.31; 8 BS-PMS beams of 30x20 K=1 024 491 -> 267 -> 213.
 // Checked on the CPU against libstdc++ over 192 000 tie-heavy replaces.
 template <typename Key>
 struct PipedHeap {
@@ -1539,7 +1539,8 @@ struct PipedHeap {
     HeapNodes<Key> h;
     int K, D;                 // size; depth of the last position
     int fpos, spos;           // lane d: positions of f and s
-    bool has_s, s_right;      // lane d: s exists in [0, K - 1); s is the right child
+    bool has_s;               // lane d: s exists in [0, K - 1)
+    Key s_add, f_mask;        // lane d: 1 if s wins a tie (it is the right child); 0 at depth D
     Key fk, sk, tk;
     uint32_t fv, sv, tv;
     int tpos;                 // lanes >= 16: the task's hole, -1 = none
@@ -1555,8 +1556,9 @@ struct PipedHeap {
         // node d of the path to position K - 1: the leading d + 1 bits of K, less 1
         fpos = lane <= D ? (K >> (D - lane)) - 1 : 0;
         spos = (fpos & 1) ? fpos + 1 : fpos - 1;
-        s_right = (fpos & 1) != 0;
         has_s = lane >= 1 && lane <= D && spos < K - 1;
+        s_add = has_s && (fpos & 1) ? 1 : 0;
+        f_mask = lane == D ? (Key)0 : ~(Key)0;
         fk = lane <= D ? h.key(fpos + 1) : (Key)0;
         fv = lane <= D ? h.val(fpos + 1) : 0u;
         sk = has_s ? h.key(spos + 1) : (Key)0;
@@ -1616,8 +1618,7 @@ struct PipedHeap {
         const uint32_t fdv = __shfl_down_sync(FULL_MASK, fv, 1), fuv = __shfl_up_sync(FULL_MASK, fv, 1),
                        sdv = __shfl_down_sync(FULL_MASK, sv, 1);
         // e: where the hole leaves the path; s(e) moves up and v sinks below it unless s(e) < v
-        const unsigned bal =
-            __ballot_sync(FULL_MASK, has_s && (lane == D || (s_right ? !(sk < fk) : fk < sk)));
+        const unsigned bal = __ballot_sync(FULL_MASK, sk + s_add > (fk & f_mask));   // no s: sk = 0
         const unsigned below = __ballot_sync(FULL_MASK, sk < vk);
         {
             Key ok;
@@ -1629,7 +1630,7 @@ struct PipedHeap {
             tpos = np;
         }
         __syncwarp();
-        const int e = bal ? __ffs(bal) - 1 : D;
+        const int e = (int)min((unsigned)(__ffs(bal) - 1), (unsigned)D);
         const bool moves = bal != 0u && !((below >> e) & 1u);
         const int hole = lane >= 16 ? tpos : (moves && lane == e ? spos : -1);
         const Kids kb = kids(hole);
@@ -1968,7 +1969,17 @@ __device__ __forceinline__ void heap_level(const StepArgs& a, int s, const HeapC
             int k = 0;
             if (size < K) {
                 const int more = min(K - size, nc);
-                for (; k < more; k++) heap_push<Key>(nodes, size++, ik[k], iv[k], lane);
+                Key xk = more ? ik[0] : (Key)0;
+                uint32_t xv = more ? iv[0] : 0u;
+                while (k < more) {
+                    // the next child is read before the push's stores
+                    const int kn = min(++k, more - 1);
+                    const Key yk = ik[kn];
+                    const uint32_t yv = iv[kn];
+                    heap_push<Key>(nodes, size++, xk, xv, lane);
+                    xk = yk;
+                    xv = yv;
+                }
                 if (size == K) {
                     heap.load(K, lane);
                     if (lane == 0) *reinterpret_cast<volatile unsigned long long*>(s_front) = heap.fk;
