@@ -204,6 +204,11 @@ struct BeamConst {
     unsigned long long* spill;
 };
 
+// The level loop's state across the fallback's call (one copy per block: every thread holds the same).
+struct LevelState {
+    int seg, t, plo, shift, recount_ok, lo, cnt, V, Vb, keff, R, Pn, w0, w1, Tb;
+};
+
 // Fixed part of the dynamic shared memory (bytes); the rest of the layout is SearchCfg's.
 constexpr int kRow = NB / 2 + 4;                  // words: 16-bit counts of two bins, then the valid children
 constexpr int kOffHist = 0;                       // u32[NB] this block's keys per bin
@@ -256,13 +261,14 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
     __shared__ BeamConst B;
     __shared__ uint4 s_pub[1];                 // min, max score bits (y, z)
     __shared__ __align__(8) unsigned long long s_bar[kMaxAhead * T / 32];   // per round and warp
+    __shared__ LevelState s_keep;
     __shared__ int s_ws[2][32];
     __shared__ int s_T, s_first, s_maxbin, s_x0, s_x1, s_mymax, s_valid, s_lcount, s_tie;
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int C = cf.cluster;
-    const unsigned rank = C > 1 ? cluster_rank() : 0u;
-    const int seg = __ldg(cf.list + blockIdx.x / (unsigned)C);
+    unsigned rank = C > 1 ? cluster_rank() : 0u;
+    int seg = __ldg(cf.list + blockIdx.x / (unsigned)C);
 
     uint32_t* const hist = reinterpret_cast<uint32_t*>(smem + kOffHist);
     uint32_t* const packed = reinterpret_cast<uint32_t*>(smem + kOffPack);
@@ -327,9 +333,10 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
     if (lane == 0)
         for (int k = 0; k < kMaxAhead; k++) bar_init(&s_bar[k * (T / 32) + warp]);
     __syncthreads();
-    const int n = B.n, S = B.S, SP = cf.stage_stride;
-    const bool usemask = B.mode != MODE_CLEAN;
-    const bool split = cf.rs * S > (64 << 10);   // children's stores in quarters
+    int n = B.n, S = B.S;
+    const int SP = cf.stage_stride;
+    bool usemask = B.mode != MODE_CLEAN;
+    bool split = cf.rs * S > (64 << 10);   // children's stores in quarters
     int P = 1, Pc = 1, lo = rank == 0 ? 0 : 1, cnt = rank == 0 ? 1 : 0;
     if (usemask)
 #pragma unroll 1
@@ -340,8 +347,8 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
     bool recount_ok = true;
     csync();   // the cluster's shared memory is initialised before any remote access
 
-    const int sv = tid / G, gl = lane % G;
-    const int gsh = (lane / G) * G;
+    int sv = tid / G, gl = lane % G;
+    int gsh = (lane / G) * G;
 
     for (int t = 0;; t++) {
         const uint32_t seed_t = B.seed + (uint32_t)t;
@@ -1021,16 +1028,41 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             }
             mn = __reduce_min_sync(FULL_MASK, mn);
             mx = __reduce_max_sync(FULL_MASK, mx);
+            // Nothing but the warps' copy phases stays in registers across the call: what does is
+            // kept in local memory for the whole level loop (84-168 bytes per thread).  us per call
+            // with and without: 15x15 K=256 1 654 -> 1 456, v1 20x15 K=1024 3 266 -> 2 932, 50x20
+            // K=4096 13 602 -> 12 425, 8 beams 17 539 -> 16 042, 100x20 8 beams 43 166 -> 39 875.
+            if (tid == 0)
+                s_keep = LevelState{seg, t, (int)plo, shift, recount_ok ? 1 : 0, lo, cnt, V, Vb, keff, R,
+                                    Pn, w0, w1, Tb};
             if (rank == 0) sorted_fallback(a.st[seg], d.K, R, V, a.keys + d.key_off, a.sel + d.sel_off, smem, mn, mx);
             csync();
             __threadfence();
+            {
+                const volatile LevelState& k = s_keep;
+                const volatile BeamConst& b = B;
+                seg = k.seg; t = k.t; plo = (uint32_t)k.plo; shift = k.shift;
+                recount_ok = k.recount_ok != 0; lo = k.lo; cnt = k.cnt; V = k.V; Vb = k.Vb; keff = k.keff; R = k.R;
+                Pn = k.Pn; w0 = k.w0; w1 = k.w1; Tb = k.Tb;
+                n = b.n; S = b.S;
+                usemask = b.mode != MODE_CLEAN;
+                split = cf.rs * S > (64 << 10);
+                asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+                lane = tid & 31;
+                warp = tid >> 5;
+                sv = tid / G;
+                gl = lane % G;
+                gsh = (lane / G) * G;
+                rank = C > 1 ? cluster_rank() : 0u;
+            }
             load_tables();
+            const SegDesc& d2 = a.segs[seg];
 #pragma unroll 1
-            for (int i = tid; i < w1 - w0; i += T) sel[i] = __ldcg(a.sel + d.sel_off + w0 + i);
+            for (int i = tid; i < w1 - w0; i += T) sel[i] = __ldcg(a.sel + d2.sel_off + w0 + i);
             if (usemask)
 #pragma unroll 1
-                for (int i = tid; i < cnt * words; i += T)
-                    masks[i] = __ldcg(a.masks + d.mask_off + (int64_t)lo * words + i);
+                for (int i = tid; i < cnt * d2.words; i += T)
+                    masks[i] = __ldcg(a.masks + d2.mask_off + (int64_t)lo * d2.words + i);
             __syncthreads();
         }
         if (keff > R) {
