@@ -13,12 +13,13 @@
 //           its candidates found (a byte compare of the ready positions' machines against the
 //           pivot machine), then a thread per candidate scores it; keys go to the block's list
 //           and are counted into 512 score bins
-//   #1      every block reads the others' counts -> V, the bin T that holds rank R, each bin's
+//   #1      every block reads the others' packed counts -> V, the bin T that holds rank R, each bin's
 //           first position; the keys of bins <= T go to the block(s) owning their bin's
 //           positions, in any order
 //   #2      keys are unique (score, slot) pairs, so a key's position is its bin's first
-//           position plus the smaller keys of the bin: counted directly in small bins, by a
-//           bitonic sort of the block's keys when a bin is large
+//           position plus the smaller keys of the bin: counted directly in small bins, within
+//           groups of equal scores in larger ones, by a bitonic sort of the block's keys when
+//           neither holds
 //
 // The bins are linear in the score bits over a range predicted from the previous level (the
 // map is monotone whatever the range, so a poor prediction costs time, not correctness): a
@@ -33,13 +34,14 @@
 // use the level kernels.)
 //
 // What bounds it: the level's chain of dependent instructions and barriers (50x20 K=4096 on
-// 16 blocks: ~32 K cycles per level, 2 770 instructions per warp, 0.45 issued per scheduler and
-// cycle), and the children's stores (an SM writes ~30 bytes per cycle to L2).  512 threads:
-// 1 024 measured 9.8 against 8.1 us per level at 15x15 K=256 (barriers and issue slots), 256
-// 12.0.  Snapshots by bulk copies: 256 of 448 bytes load in 2 350 cycles, by 16-byte cp.async
-// in 4 280.  GB300, us per call, level kernels -> this: 15x15 K=256 3 332 -> 1 873; v1 20x15
-// K=1024 6 836 -> 3 459; v1 20x15 K=16384 75 838 -> 22 437; 50x20 K=4096 24 288 -> 14 966, 8 beams
-// 28 182 -> 20 846; 100x20 K=4096 8 beams 66 166 -> 48 314.
+// 16 blocks: ~25 K cycles per level), the blocks' differences at barrier #1, and for wide
+// shares of long lists the children's stores (an SM writes ~30 bytes per cycle to L2).  512
+// threads: 1 024 measured 9.8 against 8.1 us per level at 15x15 K=256 (barriers and issue
+// slots), 256 12.0.  Snapshots by bulk copies: 256 of 448 bytes load in 2 350 cycles, by
+// 16-byte cp.async in 4 280.  GB300, us per call, level kernels -> this: 15x15 K=256 3 332 ->
+// 1 456; v1 20x15 K=1024 6 836 -> 2 932; v1 20x15 K=16384 64 083-75 838 -> 22 000-23 400;
+// 50x20 K=4096 24 288 -> 12 425, 8 beams 28 182 -> 16 042; 100x20 K=4096 8 beams 66 166 ->
+// 39 875.
 #include <algorithm>
 #include <mutex>
 #include <type_traits>
@@ -1255,10 +1257,11 @@ cudaError_t search_device(SearchDevice& out)
     return cudaSuccess;
 }
 
-// Fitted to single beams on GB300, us per level over survivors per block (v2, 20x20): one block
-// 64: 5.8, 128: 6.4, 256: 8.1, 384: 10.5, 512: 14.6, 1 024: 27.7, 2 048: 50.6; 2 blocks +1.9, 16
-// +3.8 (barriers); lists of 50 / 100 jobs cost 1.4 / 2 times as much per survivor; v1 also
-// writes the scored children (1 024: 62.4).
+// Fitted to single beams on GB300 (before the last 15 % came off every size: the choice needs
+// ratios only), us per level over survivors per block (v2, 20x20): one block 64: 5.8, 128: 6.4,
+// 256: 8.1, 384: 10.5, 512: 14.6, 1 024: 27.7, 2 048: 50.6; 2 blocks +1.9, 16 +3.8 (barriers);
+// lists of 50 / 100 jobs cost 1.4 / 2 times as much per survivor; v1 also writes the scored
+// children (1 024: 62.4).
 double search_level_us(int n, int K, bool v1, int C)
 {
     const double at[] = {64, 128, 256, 384, 512}, cost[] = {0, 0.7, 2.6, 5.2, 9.3}, slots[] = {0.9, 2.0, 4.8, 7.4, 10.0};
