@@ -87,6 +87,13 @@ struct SearchLay {
     }
 };
 
+// A survivor's entry (filler flag | parent rank << 7 | ready position or branch) names one of the
+// P parents and a place in a list of n: only then are its copies inside the beam's buffers.
+__host__ __device__ __forceinline__ bool search_entry_ok(uint32_t e, int P, int n)
+{
+    return ((e & ~kFillerFlag) >> 7) < (uint32_t)P && (e & 127u) < (uint32_t)n;
+}
+
 // One launch: its beams, blocks per beam, lanes per survivor and shared-memory layout.
 struct SearchCfg {
     const int32_t* list;        // the launch's beams

@@ -196,7 +196,7 @@ constexpr int kRecountBin = 1536;
 // What a block keeps of its beam.  In shared memory, not registers: the level loop's live
 // state would otherwise spill, and local memory does not fit the L1 the shared memory leaves.
 struct BeamConst {
-    int n, m, N, K, mode, words, S, bound, off_jr, off_op, off_mc, off_hdr, WL, P;
+    int n, m, N, K, mode, words, S, bound, off_jr, off_op, off_mc, off_hdr, WL, P, parents;   // parents: entries `sel` may name
     uint32_t seed, paths;
     float inv_m, inv_s16;
     int levels;
@@ -320,6 +320,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
         B.inv_s16 = 1.0f / (float)(L.bytes >> 4);
         B.WL = (((d.n + 3) >> 2) + G - 1) / G;   // ready-position words per lane
         B.P = 1;
+        B.parents = 0;
         B.paths = 0;
         B.levels = 0;
         B.expanded = B.slots = B.mat = 0;
@@ -374,7 +375,9 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             auto piece = [&](int i, const uint4*& from, uint4*& to) {
                 const int x = (int)(((float)i + 0.5f) * B.inv_s16), q = i - x * (S >> 4);
                 const uint32_t e = sel[x] & ~kFillerFlag;
-                from = reinterpret_cast<const uint4*>(B.slot_base + (int64_t)((int)(e >> 7) * n + (int)(e & 127u)) * S) + q;
+                // (an entry that is no survivor is reported in the step below)
+                const int c = min((int)(e >> 7), B.parents - 1), b = min((int)(e & 127u), n - 1);
+                from = reinterpret_cast<const uint4*>(B.slot_base + (int64_t)(c * n + b) * S) + q;
                 to = reinterpret_cast<uint4*>(B.beam0 + (lo + x) * S) + q;
             };
 #pragma unroll 1
@@ -402,7 +405,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
         if (ahead) {
             for (int rd = 0; rd < rounds; rd++) {
                 const int rl = rd * cf.rs + sv;
-                const bool head = gl == 0 && sv < cf.rs && rl < cnt;
+                const bool head = gl == 0 && sv < cf.rs && rl < cnt && search_entry_ok(sel[rl], B.parents, n);
                 const uint32_t heads = __ballot_sync(FULL_MASK, head);
                 unsigned long long* bar = &s_bar[rd * (T / 32) + warp];
                 if (lane == 0 && heads) bar_expect(bar, __popc(heads) * S);
@@ -426,7 +429,14 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             uint8_t* const mcb = sb + B.off_mc;
             uint4* const hdr = reinterpret_cast<uint4*>(sb + B.off_hdr);   // r | ns << 16, cmax, lineage, stamp
             if (t > 0) {
-                if (act) e = sel[rl];
+                if (act) {
+                    e = sel[rl];
+                    if (!search_entry_ok(e, B.parents, n)) {
+                        // no survivor: it takes no part
+                        if (gl == 0) atomicOr(&a.st[seg].status, kStatusBadSelect);
+                        act = false;
+                    }
+                }
                 if (V1) {
                     if (act) {
                         const int c = (int)((e & ~kFillerFlag) >> 7);
@@ -834,6 +844,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             B.levels += 1;
             B.mat += lastlv ? 0 : keff;
             B.P = keff;
+            B.parents = P;
             const bool large = V > kStageKeys || B.K > kLsdMax;
             if (R > 0 && !lastlv) B.paths |= large ? kPathLarge : (cf.wide && C > 1 && V > kClusterMinKeys ? kPathCluster : kPathDirect);
         }

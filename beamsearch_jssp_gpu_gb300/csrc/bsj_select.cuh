@@ -702,6 +702,8 @@ __device__ __forceinline__ void bitonic_in_thread(unsigned long long (&x)[E], in
 template <int E>
 static __device__ void block_bitonic_reg(unsigned long long (&x)[E], unsigned long long* xs)
 {
+    // the longest in-thread distance below is 16: at 64 keys per thread padding ends up among the keys
+    static_assert(E <= 32, "block_bitonic_reg sorts at most 32 keys per thread");
     const int t = threadIdx.x, lane = t & 31;
     const int N = E * kSelectThreads;
     for (int k = 2; k <= N; k <<= 1) {
