@@ -94,6 +94,13 @@ __host__ __device__ __forceinline__ bool search_entry_ok(uint32_t e, int P, int 
     return ((e & ~kFillerFlag) >> 7) < (uint32_t)P && (e & 127u) < (uint32_t)n;
 }
 
+// Position i is one of the ready list's (first header word: list length | operations done << 16).
+// Applied past its end, an operation would shorten an empty list to 65 535 entries.
+__host__ __device__ __forceinline__ bool search_position_ok(int i, uint32_t header)
+{
+    return i >= 0 && i < (int)(header & 0xFFFFu);
+}
+
 // One launch: its beams, blocks per beam, lanes per survivor and shared-memory layout.
 struct SearchCfg {
     const int32_t* list;        // the launch's beams

@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                         }
                         ii = found;
                     }
-                    const bool apply = act && ii >= 0;
+                    const bool apply = act && search_position_ok(ii, h.x);
                     int opx = 0, opl = 0, mcx = 0, mcl = 0, jrl = 0, fin = 0, last = 0;
                     uint32_t o = 0;
                     if (apply) {
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                         for (int q = gl; q < (S >> 4); q += G) reinterpret_cast<uint4*>(sb)[q] = __ldcg(s4 + q);
                         if (gl == 0) {
                             B.hist[(t - 1) * B.K + r] = kMark;
-                            if (B.mode == MODE_CLEAN) atomicOr(&a.st[seg].status, kStatusBadSelect);
+                            if (B.mode == MODE_CLEAN || !(e & kFillerFlag)) atomicOr(&a.st[seg].status, kStatusBadSelect);
                         }
                     }
                     __syncwarp();

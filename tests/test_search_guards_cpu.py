@@ -1,6 +1,7 @@
 """Guards of the selection and of the resident search that need no GPU: the register sort
 refuses more keys per thread than it can order, and an entry of the survivor list is taken
-for a survivor only if it names a parent and a place in its list."""
+for a survivor only if it names a parent and a place in its list, and applied only inside
+the parent's present list."""
 import os
 import subprocess
 
@@ -16,7 +17,8 @@ int main()
 {
     unsigned e;
     int P, n;
-    while (std::scanf("%u %d %d", &e, &P, &n) == 3) std::printf("%d\\n", bsj::search_entry_ok(e, P, n) ? 1 : 0);
+    while (std::scanf("%u %d %d", &e, &P, &n) == 3)
+        std::printf("%d\\n", (n > 0 ? bsj::search_entry_ok(e, P, n) : bsj::search_position_ok(P, e)) ? 1 : 0);
 }
 """
 
@@ -42,6 +44,8 @@ def test_survivor_entries(tmp_path):
     cases = [(0, 1, 1, 1), (127, 1, 128, 1), (127, 1, 127, 0), (128, 1, 128, 0), (4095 << 7 | 49, 4096, 50, 1),
              (4095 << 7 | 50, 4096, 50, 0), (4096 << 7, 4096, 50, 0), (filler | 16383 << 7 | 3, 16384, 4, 1),
              (filler | 16384 << 7, 16384, 4, 0), (0xFFFFFFFF, 16384, 128, 0), (0x7FFFFFFF, 16384, 128, 0), (0, 0, 5, 0)]
+    # a list's header, a position in it (told apart by the last number)
+    cases += [(3, 2, 0, 1), (3, 3, 0, 0), (3, -1, 0, 0), (7 << 16, 0, 0, 0), (7 << 16 | 1, 0, 0, 1)]
     text = "\n".join(f"{e} {P} {n}" for e, P, n, _ in cases)
     got = subprocess.run([str(tmp_path / "t")], input=text, capture_output=True, text=True).stdout.split()
     assert [int(x) for x in got] == [c[3] for c in cases]
