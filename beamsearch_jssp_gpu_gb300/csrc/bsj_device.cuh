@@ -100,6 +100,8 @@ struct SegDesc {
     int32_t nq;         // ceil(n / 32): 32-lane groups a warp needs for the ready list
     int32_t kcnt_off;   // index of this beam's first per-chunk key count
     int32_t narrow_keys;  // ICH/PMS: the instance's total duration is at most kNarrowTotal
+    int32_t unit;       // greatest common divisor of the durations (1 if all are 0)
+    float slack;        // 0.08 of their mean: how far past the kept range the next level's bins reach
     int64_t beam_off[2];  // byte offsets of the two beam buffers
     int64_t slot_off;     // byte offset of the v1 child-slot buffer
     int64_t key_off;      // u64 index: candidate keys of the current level

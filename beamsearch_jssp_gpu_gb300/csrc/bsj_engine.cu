@@ -19,6 +19,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <numeric>
 #include <string>
 #include <vector>
 
@@ -195,11 +196,19 @@ bsj_status validate_instance(bsj_context* ctx, const bsj_instance& in)
     return BSJ_OK;
 }
 
-int32_t narrow_keys(const bsj_instance& in)
+// What a descriptor holds of its instance's durations.
+void describe_durations(const bsj_instance& in, SegDesc& d)
 {
+    const int64_t count = (int64_t)in.n * in.m;
     int64_t total = 0;
-    for (int64_t q = 0; q < (int64_t)in.n * in.m; q++) total += in.duration[q];
-    return total <= kNarrowTotal ? 1 : 0;
+    int32_t unit = 0;
+    for (int64_t q = 0; q < count; q++) {
+        total += in.duration[q];
+        if (unit != 1) unit = std::gcd(unit, in.duration[q]);
+    }
+    d.narrow_keys = total <= kNarrowTotal ? 1 : 0;
+    d.unit = std::max(unit, 1);
+    d.slack = 0.08f * (float)total / (float)count;
 }
 
 std::string shape_key(int ninst, const bsj_instance* insts, int nbeams, const bsj_beam* beams);
@@ -508,7 +517,7 @@ bsj_status plan_build(bsj_context* ctx, int ninst, const bsj_instance* insts, in
         d.sbytes = (int)align_up((size_t)d.off_hdr + 16, 16);
         d.words = (d.n + 31) / 32;
         d.auxbytes = (int)align_up((size_t)(4 + 6 * d.n), 16);
-        d.narrow_keys = narrow_keys(in);
+        describe_durations(in, d);
         d.group = gid[b];
         d.op_off = inst_off[bm.instance];
         d.nq = nq_class(d.n);
@@ -979,7 +988,7 @@ bsj_status plan_refresh(bsj_plan* p, int ninst, const bsj_instance* insts, const
     for (int si = 0; si < p->nseg; si++) {
         const bsj_beam& bm = beams[p->perm[si]];
         p->segs[si].seed = bm.seed;
-        p->segs[si].narrow_keys = narrow_keys(insts[bm.instance]);
+        describe_durations(insts[bm.instance], p->segs[si]);
         SegState st{};
         st.P = 1;
         st.bound = bm.best_known;

@@ -64,14 +64,29 @@ size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 // (duration << 8) | machine per op; an invalid entry is replaced by machine 0 / duration 0
 // (so no kernel indexes outside the instance) and flags the beam state.  Durations whose
 // sum reaches 2^31-1 would wrap the int32 makespans, so then the whole table is zeroed
-// and the state flagged the same way.
-__global__ void k_noalloc_pack(const int32_t* machine, const int32_t* duration, int count, int m,
-                               uint32_t* ops, SegState* st)
+// and the state flagged the same way.  Fills the descriptor's unit and slack.
+constexpr int kPackThreads = 256;
+
+__device__ int gcd_of(int a, int b)
+{
+    while (b) {
+        const int r = a % b;
+        a = b;
+        b = r;
+    }
+    return a;
+}
+
+__global__ void __launch_bounds__(kPackThreads) k_noalloc_pack(const int32_t* machine, const int32_t* duration,
+                                                               int count, int m, uint32_t* ops, SegState* st,
+                                                               SegDesc* desc)
 {
     __shared__ unsigned long long total;
+    __shared__ int part[kPackThreads / 32];
     if (threadIdx.x == 0) total = 0;
     __syncthreads();
     bool bad = false;
+    int unit = 0;
     unsigned long long local = 0;
     for (int q = threadIdx.x; q < count; q += blockDim.x) {
         int mc = machine[q], du = duration[q];
@@ -81,10 +96,18 @@ __global__ void k_noalloc_pack(const int32_t* machine, const int32_t* duration, 
             du = 0;
         }
         local += (unsigned long long)du;
+        if (unit != 1) unit = gcd_of(unit, du);
         ops[q] = ((uint32_t)du << 8) | (uint32_t)mc;
     }
     atomicAdd(&total, local);
+    for (int o = 16; o > 0; o >>= 1) unit = gcd_of(unit, __shfl_xor_sync(0xFFFFFFFFu, unit, o));
+    if (threadIdx.x % 32 == 0) part[threadIdx.x / 32] = unit;
     __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kPackThreads / 32; w++) unit = gcd_of(unit, part[w]);
+        desc->unit = max(unit, 1);
+        desc->slack = 0.08f * (float)total / (float)count;
+    }
     const bool overflow = total >= 0x7FFFFFFFull;
     if (overflow)
         for (int q = threadIdx.x; q < count; q += blockDim.x) ops[q] = 0u;
@@ -268,8 +291,9 @@ extern "C" bsj_status bsj_solve_noalloc(int32_t n, int32_t m, const int32_t* d_m
                                     reinterpret_cast<int32_t*>(base + o_group));
     if (cudaGetLastError() != cudaSuccess) return BSJ_ERR_CUDA;
     if (cudaMemsetAsync(a.beam_pool, 0, beam_bytes, s) != cudaSuccess) return BSJ_ERR_CUDA;
-    k_noalloc_pack<<<1, 256, 0, s>>>(d_machine, d_duration, d.N, m, reinterpret_cast<uint32_t*>(base + o_ops),
-                                     reinterpret_cast<SegState*>(base + o_state));
+    k_noalloc_pack<<<1, kPackThreads, 0, s>>>(d_machine, d_duration, d.N, m, reinterpret_cast<uint32_t*>(base + o_ops),
+                                     reinterpret_cast<SegState*>(base + o_state),
+                                     reinterpret_cast<SegDesc*>(base + o_seg));
     if (cudaGetLastError() != cudaSuccess) return BSJ_ERR_CUDA;
     if (launch_noise_table(const_cast<float*>(a.noise), nullptr, s) != cudaSuccess) return BSJ_ERR_CUDA;
     if (blocks) {

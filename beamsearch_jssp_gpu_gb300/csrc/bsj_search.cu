@@ -23,9 +23,10 @@
 //
 // The bins are linear in the score bits over a range predicted from the previous level (the
 // map is monotone whatever the range, so a poor prediction costs time, not correctness): a
-// level whose largest bin comes out too large is counted again over its exact range.  Levels
-// whose bins still do not fit the blocks' buffers (thousands of tied scores) are dumped to
-// global memory in slot order and sorted by the one-block routes of the level kernels.
+// level whose largest bin comes out too large, or whose last survivor lies past the range, is
+// counted again up to that survivor's bin, with linear bins and then with bins for tied scores
+// (TieMap).  Levels whose bins still do not fit the blocks' buffers are dumped to global memory in
+// slot order and sorted by the one-block routes of the level kernels.
 //
 // A snapshot is stored by ready position, not by job: position i holds the finish time of
 // its job's last operation, the operation index and its machine, so that a level needs no
@@ -61,6 +62,10 @@ static_assert(NB == T, "one bin per thread in the bin scan");
 // ops in shared memory: (duration << 8) | last-operation-of-its-job flag | machine
 constexpr uint32_t kLastOp = 0x80u;
 constexpr uint32_t kNoKey = 0xFFFFFFFFu;   // score bits of a pruned child
+// a key: score bits << 32 | bin << kSlotBits | slot.  Bins are monotone in (score, slot), so keys
+// order as without them.
+constexpr uint32_t kSlotMask = (1u << kSlotBits) - 1u;
+static_assert(NB <= 1 << (32 - kSlotBits), "bin and slot share a word");
 
 __device__ __forceinline__ void st_peer32(const void* p, unsigned rank, uint32_t v)
 {
@@ -166,7 +171,7 @@ __device__ void sort_window_e(unsigned long long* src, unsigned long long* xs, i
 #pragma unroll
     for (int e = 0; e < E; e++) {
         const int i = t * E + e, p = x0 + i;
-        if (i < count && p >= w0 && p < w1) sel[p - w0] = (uint32_t)x[e];
+        if (i < count && p >= w0 && p < w1) sel[p - w0] = (uint32_t)x[e] & kSlotMask;
     }
 }
 
@@ -192,6 +197,14 @@ constexpr int kTieMax = 1024;
 // a bin larger than kRecountBin: the level is counted again over its exact score range, which costs
 // a pass over the keys and two barriers.  384: 14.0 at 50x20 K=4096; 768 and 1 536: 13.5.
 constexpr int kRecountBin = 1536;
+constexpr int kMaxRecounts = 3;
+// Tie bins follow a level whose ranking was slow: one that sorted a block's window, or whose largest
+// group of equal scores had more than kTieSlow keys.  ms per call, 50x20 K=4096, durations
+// U[1, 99] | x 1 000: 384: 12.28 | 16.8, 192: 12.29 | 15.8, 96: 12.42 | 15.8.  They stay for 2, 4, ..
+// kTieStay levels, as long as linear bins fail each time between (a tie bin costs a division and a
+// pass over the keys: on every level of U[1, 99], 14.1).
+constexpr int kTieSlow = 192;
+constexpr int kTieStay = 64;
 
 // What a block keeps of its beam.  In shared memory, not registers: the level loop's live
 // state would otherwise spill, and local memory does not fit the L1 the shared memory leaves.
@@ -199,7 +212,8 @@ struct BeamConst {
     int n, m, N, K, mode, words, S, bound, off_jr, off_op, off_mc, off_hdr, WL, P, parents;   // parents: entries `sel` may name
     uint32_t seed, paths;
     float inv_m, inv_s16;
-    int levels;
+    int levels, unit;   // unit: greatest common divisor of the durations
+    float slack;        // 0.08 of the mean duration
     long long expanded, slots, mat;
     uint8_t *beam0, *beam1, *slot_base;
     uint32_t* hist;
@@ -208,8 +222,57 @@ struct BeamConst {
 
 // The level loop's state across the fallback's call (one copy per block: every thread holds the same).
 struct LevelState {
-    int seg, t, plo, shift, recount_ok, lo, cnt, V, Vb, keff, R, Pn, w0, w1, Tb;
+    int seg, t, recount_ok, tm, lo, cnt, V, Vb, keff, R, Pn, w0, w1, Tb;
 };
+
+// Bins of a level with many tied scores.  Scores of one makespan c lie a few ulps apart (the noise),
+// those of the next makespan thousands of ulps further: linear bins that span a few makespans put
+// all of one into one bin.  These give every makespan of the window [c0, c0 + nc) (in units of the
+// durations' common divisor) q bins: a bin for each of the nq scores c can have, in nsl parts
+// by slot; or q parts of the noise's range where it has more scores than that.  The map
+// is monotone in (score, slot) whatever its parameters: c is a rounded multiple of the score, the
+// rest a difference to one number per c, and only keys of one score are told apart by slot.
+// GB300, ms per call, one-block route or sorted windows -> tie bins (level kernels): 50x20 K=4096,
+// durations 1: 49.5 -> 13.1 (35.5), 1..5: 53.7 -> 12.0 (23.4), 1..20: 28.8 -> 12.6 (23.6); 20x15
+// K=1024, 1: 6.7 -> 2.6 (5.7), 1..2: 5.8 -> 4.1 (5.3); K=16384, 1..5: 34.0 -> 9.3 (28.3).
+struct TieMap {
+    int c0, nc, q, nq, nsl, unit;
+    float per, ns, oscale, sscale;   // oscale: noise parts per unit of score, 0 = a bin per score
+};
+
+__device__ __forceinline__ int tie_bin(const TieMap& m, uint32_t sc, uint32_t slot)
+{
+    const float f = __uint_as_float(sc);
+    const int c = __float2int_rn(__fmul_rn(f, m.per)), g = c - m.c0;
+    if (g < 0) return 0;
+    if (g >= m.nc) return NB - 1;
+    const float base = __fdiv_rn(__int2float_rn((int)((uint32_t)c * (uint32_t)m.unit)), m.ns);
+    if (m.oscale > 0.0f) return g * m.q + min(max((int)__fmul_rn(__fsub_rn(f, base), m.oscale), 0), m.nq - 1);
+    const int o = (int)(sc - __float_as_uint(base));
+    if (o < 0) return g * m.q;
+    if (o >= m.nq) return g * m.q + m.q - 1;
+    return g * m.q + o * m.nsl + min((int)__fmul_rn(__int2float_rn((int)slot), m.sscale), m.nsl - 1);
+}
+
+// The map of makespans c0 .. c0 + nc - 1 (nc <= NB), scores from flo on, P parents.
+__device__ __forceinline__ void tie_map(TieMap& m, int c0, int nc, int unit, float ns, float flo, int P)
+{
+    const int most = NB / nc;
+    // noise of up to 0.000000999 in steps of an ulp of the lowest score
+    const float ulp = __uint_as_float(__float_as_uint(flo) + 1u) - flo;
+    const int scores = 1 + (int)fminf(0.999e-6f / fmaxf(ulp, 1e-12f) + 0.5f, 1e6f);
+    const int nq = min(scores, most), nsl = most / nq;
+    m.c0 = c0;
+    m.nc = nc;
+    m.unit = unit;
+    m.ns = ns;
+    m.per = __fdiv_rn(ns, (float)unit);
+    m.oscale = scores > most ? 1e6f * (float)most : 0.0f;
+    m.nq = nq;
+    m.nsl = nsl;
+    m.q = nq * nsl;
+    m.sscale = (float)nsl / (float)(P << 7);
+}
 
 // Fixed part of the dynamic shared memory (bytes); the rest of the layout is SearchCfg's.
 constexpr int kRow = NB / 2 + 4;                  // words: 16-bit counts of two bins, then the valid children
@@ -264,8 +327,12 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
     __shared__ uint4 s_pub[1];                 // min, max score bits (y, z)
     __shared__ __align__(8) unsigned long long s_bar[kMaxAhead * T / 32];   // per round and warp
     __shared__ LevelState s_keep;
+    __shared__ TieMap s_tm[2];
     __shared__ int s_ws[2][32];
     __shared__ int s_T, s_first, s_maxbin, s_x0, s_x1, s_mymax, s_valid, s_lcount, s_tie;
+    __shared__ int s_slow;             // ranking the last level with linear bins was slow
+    __shared__ uint4 s_lin;            // score bins: plo, shift, tie; levels left with tie bins | the last stay << 16
+    __shared__ int s_any;              // s_slow of some block
 
     int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int C = cf.cluster;
@@ -316,6 +383,8 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
         B.S = L.bytes; B.off_jr = L.off_jr; B.off_op = L.off_op; B.off_mc = L.off_mc; B.off_hdr = L.off_hdr;
         B.bound = a.st[seg].bound;
         B.seed = d.seed;
+        B.unit = d.unit;
+        B.slack = d.slack;
         B.inv_m = 1.0f / (float)d.m;
         B.inv_s16 = 1.0f / (float)(L.bytes >> 4);
         B.WL = (((d.n + 3) >> 2) + G - 1) / G;   // ready-position words per lane
@@ -331,6 +400,8 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
         B.spill = cf.spill + d.key_off;
         s_valid = 0;
         s_lcount = 0;
+        s_slow = 0;
+        s_lin = make_uint4(0u, 21u, 0u, 1u << 16);
     }
     load_tables();
     if (lane == 0)
@@ -345,9 +416,8 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
 #pragma unroll 1
         for (int i = tid; i < cnt * B.words; i += T) masks[i] = 0u;
     uint32_t phase = 0;
-    uint32_t plo = 0;     // score bins of this level: bin = (score bits - plo) >> shift, clamped
-    int shift = 21;
     bool recount_ok = true;
+    int tm = 0;           // the level's tie bins are s_tm[tm]'s
     csync();   // the cluster's shared memory is initialised before any remote access
 
     int sv = tid / G, gl = lane % G;
@@ -355,6 +425,10 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
 
     for (int t = 0;; t++) {
         const uint32_t seed_t = B.seed + (uint32_t)t;
+        // score bins: bin = (score bits - plo) >> shift, clamped, or tie bins
+        uint32_t plo = s_lin.x;
+        int shift = (int)s_lin.y;
+        bool tie = s_lin.z != 0u;
         const bool lastlv = t == B.N - 1;
         const int rounds = Pc <= cf.rs ? 1 : (Pc + cf.rs - 1) / cf.rs;   // the same in every block
         // entries past list_cap live in global memory
@@ -362,10 +436,11 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
         auto lput = [&](int i, unsigned long long v) {
             if (i < cf.list_cap) list[i] = v; else B.spill[(int64_t)lo * n + i] = v;
         };
-        auto bin_of = [&](uint32_t sc) {
+        auto linear_bin = [&](uint32_t sc) {
             const uint32_t b = sc < plo ? 0u : (sc - plo) >> shift;
-            return (int)(b < (uint32_t)NB ? b : (uint32_t)(NB - 1));
+            return b < (uint32_t)NB ? b : (uint32_t)(NB - 1);
         };
+        auto bin_of = [&](unsigned long long k) { return (int)((uint32_t)k >> kSlotBits); };
 
         // ---- v1: survivors are copies of child slots, which this level's children overwrite.
         // With one round per block they are all in shared memory before the first is
@@ -636,8 +711,9 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                         const float q = __fdiv_rn(__int2float_rn(cm), __int_as_float(f.z));
                         const uint32_t sc = __float_as_uint(
                             __fadd_rn(q, noise[noise_hash(seed_t, (uint32_t)r2, (uint32_t)b) % 1000u]));
-                        key = ((unsigned long long)sc << 32) | ((uint32_t)r2 << 7) | (uint32_t)(V1 ? b : i);
-                        atomicAdd(&hist[bin_of(sc)], 1u);
+                        const uint32_t bin = linear_bin(sc);
+                        key = ((unsigned long long)sc << 32) | (bin << kSlotBits) | ((uint32_t)r2 << 7) | (uint32_t)(V1 ? b : i);
+                        if (!tie) atomicAdd(&hist[bin], 1u);
                         if (usemask) atomicOr(&masks[(rd * cf.rs + sv2) * B.words + (b >> 5)], 1u << (b & 31));
                         if (lastlv && f.w == B.N) {
                             const int job = (int)(((float)opx + 0.5f) * B.inv_m);
@@ -717,11 +793,25 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
 
         // ---- selection: V, threshold bin, positions
         int V, Vb, keff, R, Pn, w0, w1, H, Tb;   // Vb: valid children of lower blocks
-        bool exact = false;
+        int tries = 0;
         int lcount;
+        uint32_t slow;   // blocks whose ranking of the last level with linear bins was slow
         for (;;) {
             __syncthreads();
             lcount = s_lcount;
+            if (tie || tries) {
+                // the keys' bins in another map than the score's linear one
+#pragma unroll 1
+                for (int i = tid; i < lcount; i += T) {
+                    const unsigned long long k = lget(i);
+                    const uint32_t sc = (uint32_t)(k >> 32), slot = (uint32_t)k & kSlotMask;
+                    if (sc == kNoKey) continue;
+                    const uint32_t bin = tie ? (uint32_t)tie_bin(s_tm[tm], sc, slot) : linear_bin(sc);
+                    lput(i, (k & ~0xFFFFFFFFull) | (bin << kSlotBits) | slot);
+                    atomicAdd(&hist[bin], 1u);
+                }
+                __syncthreads();
+            }
             uint32_t lower = 0, tot = 0;   // of bin tid
             if (C > 1) {
                 // counts above 16 bits saturate; such a bin never fits the buffers, and V is exact
@@ -730,7 +820,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                     reinterpret_cast<uint2*>(hist)[tid] = make_uint2(0u, 0u);
                     packed[tid] = min(c.x, 0xFFFFu) | (min(c.y, 0xFFFFu) << 16);
                 } else if (tid == NB / 2) {
-                    packed[NB / 2] = (uint32_t)s_valid;
+                    packed[NB / 2] = (uint32_t)s_valid | (uint32_t)s_slow << 24;
                 }
                 csync();   // #1
                 for (int x = tid; x < C * (kRow / 4); x += T) {
@@ -746,13 +836,16 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                     tot += (col[q * kRow] >> half) & 0xFFFFu;
                 }
                 const uint32_t pv = lane < C ? rows[lane * kRow + NB / 2] : 0u;
-                V = (int)__reduce_add_sync(FULL_MASK, pv);
-                Vb = (int)__reduce_add_sync(FULL_MASK, lane < (int)rank ? pv : 0u);
+                const uint32_t sum = __reduce_add_sync(FULL_MASK, pv);
+                V = (int)(sum & 0xFFFFFFu);
+                slow = sum >> 24;
+                Vb = (int)(__reduce_add_sync(FULL_MASK, lane < (int)rank ? pv : 0u) & 0xFFFFFFu);
             } else {
                 tot = hist[tid];
                 hist[tid] = 0u;
                 V = s_valid;
                 Vb = 0;
+                slow = (uint32_t)s_slow;
             }
             const int t0 = (int)tot, b0 = block_exclusive(t0, s_ws[0], lane, warp);
             keff = usemask ? min(P * n, B.K) : min(V, B.K);
@@ -789,15 +882,18 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             __syncthreads();
             H = s_maxbin;
             Tb = s_T;
-            const bool coarse = H > kRecountBin || Pn + 2 * H > cf.buf_cap;
-            if (!coarse || exact || (!recount_ok && Pn + 2 * H <= cf.buf_cap)) {
-                // a recount that did not help (ties): no more of them for this beam while it lasts
-                if (exact) recount_ok = !coarse;
+            // too coarse, or a range that ends below the last survivor (its bin holds all that lie past it)
+            const bool fit = Pn + 2 * H <= cf.buf_cap;
+            const bool coarse = H > kRecountBin || !fit || (tries == 0 && Tb == NB - 1 && H > kPlainBinMax);
+            if (!coarse || tries == (recount_ok ? kMaxRecounts : 1) || (fit && (tries > 1 || !recount_ok))) {
+                // recounts that did not help: hardly any more of them for this beam while it lasts
+                if (tries) recount_ok = !coarse;
                 else if (!coarse) recount_ok = true;
                 break;
             }
-            // ---- the predicted bins are too coarse here: the level's exact score range, again
-            exact = true;
+            // ---- again, over the range from the level's lowest score to the bin of the last
+            // survivor: linear bins, then (or at once, if the last level had them) tie bins
+            tries++;
             uint32_t mn = 0xFFFFFFFFu, mx = 0u;
 #pragma unroll 1
             for (int i = tid; i < lcount; i += T) {
@@ -828,14 +924,31 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                 mn = w.y;
                 mx = w.z;
             }
-            plo = __reduce_min_sync(FULL_MASK, mn);
+            mn = __reduce_min_sync(FULL_MASK, mn);
             mx = __reduce_max_sync(FULL_MASK, mx);
-            const int nbits = mx > plo ? 32 - __clz(mx - plo) : 0;
-            shift = nbits > kSearchBinBits ? nbits - kSearchBinBits : 0;
-#pragma unroll 1
-            for (int i = tid; i < lcount; i += T) {
-                const uint32_t sc = (uint32_t)(lget(i) >> 32);
-                if (sc != kNoKey) atomicAdd(&hist[bin_of(sc)], 1u);
+            const bool was = tie;
+            if (!was && Tb < NB - 1)
+                mx = (uint32_t)min((unsigned long long)mx, plo + ((unsigned long long)(Tb + 1) << shift) - 1);
+            if (was || tries > 1) {
+                const float ns = (float)(t + 1), per = __fdiv_rn(ns, (float)B.unit);
+                const int c0 = __float2int_rn(__uint_as_float(mn) * per);
+                int c1 = __float2int_rn(__uint_as_float(mx) * per);
+                if (was && Tb < NB - 1) c1 = min(c1, s_tm[tm].c0 + Tb / s_tm[tm].q);
+                tie = (uint32_t)(c1 - c0) < (uint32_t)NB;
+                if (tie) {
+                    tm ^= 1;
+                    if (tid == 0) tie_map(s_tm[tm], c0, c1 - c0 + 1, B.unit, ns, __uint_as_float(mn), P);
+                }
+            }
+            if (!tie) {
+                plo = mn;
+                const int nbits = mx > plo ? 32 - __clz(mx - plo) : 0;
+                shift = nbits > kSearchBinBits ? nbits - kSearchBinBits : 0;
+            }
+            if (tid == T - 32) {
+                s_lin.x = plo;
+                s_lin.y = (uint32_t)shift;
+                s_lin.z = tie ? 1u : 0u;
             }
         }
         if (tid == 0) {
@@ -845,6 +958,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             B.mat += lastlv ? 0 : keff;
             B.P = keff;
             B.parents = P;
+            s_any = (int)slow;
             const bool large = V > kStageKeys || B.K > kLsdMax;
             if (R > 0 && !lastlv) B.paths |= large ? kPathLarge : (cf.wide && C > 1 && V > kClusterMinKeys ? kPathCluster : kPathDirect);
         }
@@ -856,9 +970,8 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
 #pragma unroll 1
             for (int i = tid; i < lcount; i += T) {
                 const unsigned long long k = lget(i);
-                const uint32_t sc = (uint32_t)(k >> 32);
-                if (sc == kNoKey) continue;
-                const int bin = bin_of(sc);
+                if ((uint32_t)(k >> 32) == kNoKey) continue;
+                const int bin = bin_of(k);
                 if (bin > Tb) continue;
                 const int p = (int)atomicAdd(&cur[bin], 1u);
                 if (C > 1) {
@@ -879,6 +992,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             }
             csync();   // #2
             const int x0 = s_x0, x1 = s_x1;
+            if (tid == 0) s_slow = 0;
             unsigned long long* const win = buf + (H - w0);   // by global position
             if (s_mymax <= kPlainBinMax) {
                 // small bins: two lanes per key count the smaller keys of its bin
@@ -889,7 +1003,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                     unsigned long long k = 0;
                     if (x < x1) {
                         k = win[x];
-                        const int bin = bin_of((uint32_t)(k >> 32));
+                        const int bin = bin_of(k);
                         f0 = (int)binbase[bin];
                         const int ft = (int)total[bin];
                         const unsigned long long* y = win + f0;
@@ -898,28 +1012,28 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                     }
                     c += __shfl_xor_sync(FULL_MASK, c, 1);
                     const int p = f0 + c;
-                    if (x < x1 && !(tid & 1) && p >= w0 && p < w1) sel[p - w0] = (uint32_t)k;
+                    if (x < x1 && !(tid & 1) && p >= w0 && p < w1) sel[p - w0] = (uint32_t)k & kSlotMask;
                 }
             } else {
                 // larger bins hold a few scores, a few ulps apart (one makespan, different
                 // noise): keys are placed by exact score within their bin, then each counts the
                 // smaller slots among its equals
                 uint32_t* const win2 = reinterpret_cast<uint32_t*>(buf + cf.buf_cap) + (H - w0);   // group, slot by position
-                const int bin0 = x0 < x1 ? bin_of((uint32_t)(win[x0] >> 32)) : 0;
-                const int nb = x0 < x1 ? bin_of((uint32_t)(win[x1 - 1] >> 32)) - bin0 + 1 : 0;
+                const int bin0 = x0 < x1 ? bin_of(win[x0]) : 0;
+                const int nb = x0 < x1 ? bin_of(win[x1 - 1]) - bin0 + 1 : 0;
                 bool ok = nb <= kSubBins;
                 if (ok) {
 #pragma unroll 1
                     for (int x = x0 + tid; x < x1; x += T) {
-                        const uint32_t sc = (uint32_t)(win[x] >> 32);
-                        ref[bin_of(sc) - bin0] = sc;   // any score of the bin
+                        const unsigned long long k = win[x];
+                        ref[bin_of(k) - bin0] = (uint32_t)(k >> 32);   // any score of the bin
                     }
                     __syncthreads();
 #pragma unroll 1
                     for (int x = x0 + tid; x < x1; x += T) {
-                        const uint32_t sc = (uint32_t)(win[x] >> 32);
-                        const int lb = bin_of(sc) - bin0;
-                        const uint32_t o = sc - ref[lb] + kSubs / 2;
+                        const unsigned long long k = win[x];
+                        const int lb = bin_of(k) - bin0;
+                        const uint32_t o = (uint32_t)(k >> 32) - ref[lb] + kSubs / 2;
                         if (o < (uint32_t)kSubs) atomicAdd(&sub[lb * kSubs + o], 1u);
                         else s_tie = 1 << 30;   // scores further apart than the table
                     }
@@ -941,14 +1055,15 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                     __syncthreads();
                     ok = s_tie <= kTieMax;
                 }
+                if (tid == 0 && !tie && (!ok || s_tie > kTieSlow)) s_slow = 1;
                 if (ok) {
 #pragma unroll 1
                     for (int x = x0 + tid; x < x1; x += T) {
                         const unsigned long long k = win[x];
                         const uint32_t sc = (uint32_t)(k >> 32);
-                        const int lb = bin_of(sc) - bin0, g = lb * kSubs + (int)(sc - ref[lb]) + kSubs / 2;
+                        const int lb = bin_of(k) - bin0, g = lb * kSubs + (int)(sc - ref[lb]) + kSubs / 2;
                         const int p = (int)atomicAdd(&sub[g], 1u);   // afterwards sub[g] is the group's end
-                        win2[p] = ((uint32_t)g << kSlotBits) | (uint32_t)k;
+                        win2[p] = ((uint32_t)g << kSlotBits) | ((uint32_t)k & kSlotMask);
                     }
                     __syncthreads();
 #pragma unroll 1
@@ -972,7 +1087,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                         }
                         c += __shfl_xor_sync(FULL_MASK, c, 1);
                         const int p = f0 + c;
-                        if (x < x1 && !(tid & 1) && p >= w0 && p < w1) sel[p - w0] = k & ((1u << kSlotBits) - 1u);
+                        if (x < x1 && !(tid & 1) && p >= w0 && p < w1) sel[p - w0] = k & kSlotMask;
                     }
                 } else {
                     sort_window(win + x0, buf, x1 - x0, x0, w0, w1, sel);
@@ -996,7 +1111,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             uint32_t mn = 0xFFFFFFFFu, mx = 0u;
             for (int i = tid; i < lcount; i += T) {
                 const unsigned long long k = lget(i);
-                const uint32_t sc = (uint32_t)(k >> 32), sl = (uint32_t)k;
+                const uint32_t sc = (uint32_t)(k >> 32), sl = (uint32_t)k & kSlotMask;
                 if (sc == kNoKey) continue;
                 mn = min(mn, sc);
                 mx = max(mx, sc);
@@ -1022,13 +1137,13 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             __syncthreads();
             for (int i = tid; i < lcount; i += T) {
                 const unsigned long long k = lget(i);
-                const uint32_t sl = (uint32_t)k;
+                const uint32_t sl = (uint32_t)k & kSlotMask;
                 if ((uint32_t)(k >> 32) == kNoKey) continue;
                 const int c = (int)(sl >> 7) - lo;
                 int p = first[c];
                 for (uint32_t w = 0; w < ((sl & 127u) >> 5); w++) p += __popc(bits[c * words + w]);
                 p += __popc(bits[c * words + ((sl & 127u) >> 5)] & ((1u << (sl & 31u)) - 1u));
-                dump[p] = k;
+                dump[p] = (k & ~0xFFFFFFFFull) | sl;
             }
             csync();
             __threadfence();
@@ -1046,7 +1161,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             // with and without: 15x15 K=256 1 654 -> 1 456, v1 20x15 K=1024 3 266 -> 2 932, 50x20
             // K=4096 13 602 -> 12 425, 8 beams 17 539 -> 16 042, 100x20 8 beams 43 166 -> 39 875.
             if (tid == 0)
-                s_keep = LevelState{seg, t, (int)plo, shift, recount_ok ? 1 : 0, lo, cnt, V, Vb, keff, R,
+                s_keep = LevelState{seg, t, recount_ok ? 1 : 0, tm, lo, cnt, V, Vb, keff, R,
                                     Pn, w0, w1, Tb};
             if (rank == 0) sorted_fallback(a.st[seg], d.K, R, V, a.keys + d.key_off, a.sel + d.sel_off, smem, mn, mx);
             csync();
@@ -1054,8 +1169,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             {
                 const volatile LevelState& k = s_keep;
                 const volatile BeamConst& b = B;
-                seg = k.seg; t = k.t; plo = (uint32_t)k.plo; shift = k.shift;
-                recount_ok = k.recount_ok != 0; lo = k.lo; cnt = k.cnt; V = k.V; Vb = k.Vb; keff = k.keff; R = k.R;
+                seg = k.seg; t = k.t; recount_ok = k.recount_ok != 0; tm = k.tm; lo = k.lo; cnt = k.cnt; V = k.V; Vb = k.Vb; keff = k.keff; R = k.R;
                 Pn = k.Pn; w0 = k.w0; w1 = k.w1; Tb = k.Tb;
                 n = b.n; S = b.S;
                 usemask = b.mode != MODE_CLEAN;
@@ -1077,6 +1191,44 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                 for (int i = tid; i < cnt * d2.words; i += T)
                     masks[i] = __ldcg(a.masks + d2.mask_off + (int64_t)lo * d2.words + i);
             __syncthreads();
+        }
+        // ---- the next level's bins: this level's kept scores, one operation later (in a warp that has
+        // no keys to rank where the share is small)
+        if (tid == T - 32 && R == 0) s_lin.z = 0u;
+        if (tid == T - 32 && R > 0) {
+            const uint4 lin = s_lin;
+            const float u = __fdividef(1.0f, (float)(t + 2));
+            // f0, f1: the scores kept.  The lowest child keeps its makespan; above, half the kept range
+            // and some more (a narrow beam's range is a few operations' differences wide, and a
+            // prediction that misses it clamps all keys into one bin)
+            float f0 = __uint_as_float(lin.x + ((uint32_t)s_first << lin.y));
+            float f1 = __uint_as_float(lin.x + (((uint32_t)Tb + 1u) << lin.y) - 1u);
+            int left = (int)(lin.w & 0xFFFFu), stay = (int)(lin.w >> 16), next_tie = 0;
+            if (lin.z | (uint32_t)s_any | (lin.w ^ (1u << 16))) {
+                // tie bins for the next levels where linear ones did not do, and for twice as many
+                // each time that they do not again
+                if (lin.z) {
+                    const TieMap& m = s_tm[tm];
+                    const float score = __fdiv_rn((float)m.unit, m.ns);
+                    f0 = (float)(m.c0 + min(s_first / m.q, m.nc)) * score;
+                    f1 = (float)(m.c0 + min(Tb / m.q, m.nc) + 1) * score;
+                }
+                if (left > 0) left--;
+                else if (lin.z || s_any) left = stay = min(2 * stay, kTieStay);
+                else stay = max(stay / 2, 1);
+                if (left > 0) {
+                    const float g0 = f0 - f0 * u, g1 = f1 + 0.5f * (f1 - f0) + B.slack * u;
+                    const float ns = (float)(t + 2), per = __fdiv_rn(ns, (float)B.unit);
+                    const int c0 = __float2int_rn(g0 * per), c1 = __float2int_rn(g1 * per);
+                    next_tie = (uint32_t)(c1 - c0) < (uint32_t)NB ? 1 : 0;
+                    if (next_tie) tie_map(s_tm[tm ^ 1], c0, c1 - c0 + 1, B.unit, ns, g0, keff);
+                }
+            }
+            const float g0 = f0 - f0 * u, g1 = f1 + 0.5f * (f1 - f0) + B.slack * u;
+            const uint32_t lo32 = __float_as_uint(g0), hi32 = __float_as_uint(g1);
+            const int nbits = hi32 > lo32 ? 32 - __clz(hi32 - lo32) : 0;
+            s_lin = make_uint4(lo32, (uint32_t)(nbits > kSearchBinBits ? nbits - kSearchBinBits : 0),
+                               (uint32_t)next_tie, (uint32_t)(left | stay << 16));
         }
         if (keff > R) {
             // ---- v1 / v2: the lowest-numbered unscored slots follow, in slot order
@@ -1108,20 +1260,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             }
             csync();
         }
-        // ---- the next level's bins: this level's kept scores, one operation later
-        if (R > 0) {
-            const uint32_t e0 = plo + ((uint32_t)s_first << shift), e1 = plo + (((uint32_t)Tb + 1u) << shift) - 1u;
-            const float f0 = __uint_as_float(e0), f1 = __uint_as_float(e1);
-            // the lowest child keeps its makespan; above, half the kept range and four units of
-            // makespan more (a narrow beam's range is a few units wide, and a prediction that
-            // misses it clamps all keys into one bin)
-            const float u = __fdividef(1.0f, (float)(t + 2));
-            const float g0 = f0 - f0 * u, g1 = f1 + 0.5f * (f1 - f0) + 4.0f * u;
-            plo = __float_as_uint(g0);
-            const uint32_t phi = __float_as_uint(g1);
-            const int nbits = phi > plo ? 32 - __clz(phi - plo) : 0;
-            shift = nbits > kSearchBinBits ? nbits - kSearchBinBits : 0;
-        }
+        tm ^= 1;
         P = keff;
         Pc = Pn;
         lo = min(w0, P);
