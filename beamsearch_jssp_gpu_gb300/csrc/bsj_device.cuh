@@ -73,6 +73,11 @@ constexpr int kSelAll = 511;
 // Routes the levels of a beam took (SegState::select_paths, OR over the levels).
 constexpr uint32_t kPathLarge = 1, kPathDirect = 2, kPathBucket = 4, kPathRadix = 8, kPathDense = 16,
                    kPathRankLsd = 32, kPathRawLsd = 64, kPathBitonic = 128, kPathCluster = 256;
+// the resident search: what its levels took (the bits above name a level's size class there), and
+// the thread blocks of a beam: bit kPathBlocks + index in kSearchSizes
+constexpr uint32_t kPathResident = 512, kPathRecount = 1024, kPathTieBins = 2048, kPathWindowSort = 4096,
+                   kPathOneBlock = 8192;
+constexpr int kPathBlocks = 16;
 // The cluster select: launched for beams of K >= kSelectClusterMinK, its route taken on
 // levels of more than kClusterMinKeys keys, 2 CTAs per beam, or 4 where K * n reaches
 // kSelectClusterWideKN (levels of ~15 K keys and more).  Measured on GB300 (ms per search):

@@ -1352,7 +1352,17 @@ static_assert(BSJ_SELECT_FORCE_LARGE == kSelForceLarge && BSJ_SELECT_NO_LARGE ==
 static_assert(BSJ_ROUTE_LARGE == kPathLarge && BSJ_ROUTE_DIRECT == kPathDirect && BSJ_ROUTE_BUCKET == kPathBucket &&
               BSJ_ROUTE_RADIX == kPathRadix && BSJ_ROUTE_DENSE == kPathDense &&
               BSJ_ROUTE_RANK_LSD == kPathRankLsd && BSJ_ROUTE_RAW_LSD == kPathRawLsd &&
-              BSJ_ROUTE_BITONIC == kPathBitonic && BSJ_ROUTE_CLUSTER == kPathCluster, "route bits of bsj.h and the kernels differ");
+              BSJ_ROUTE_BITONIC == kPathBitonic && BSJ_ROUTE_CLUSTER == kPathCluster && BSJ_ROUTE_RESIDENT == kPathResident &&
+              BSJ_ROUTE_RECOUNT == kPathRecount && BSJ_ROUTE_TIE_BINS == kPathTieBins &&
+              BSJ_ROUTE_WINDOW_SORT == kPathWindowSort && BSJ_ROUTE_ONE_BLOCK == kPathOneBlock,
+              "route bits of bsj.h and the kernels differ");
+constexpr bool block_bits_agree()
+{
+    for (int k = 0; k < (int)(sizeof(kSearchSizes) / sizeof(kSearchSizes[0])); k++)
+        if (BSJ_ROUTE_BLOCKS(kSearchSizes[k]) != 1 << (kPathBlocks + k)) return false;
+    return true;
+}
+static_assert(block_bits_agree(), "block bits of bsj.h and the kernels differ");
 
 bsj_status bsj_plan_set_select_route(bsj_plan* p, int32_t flags)
 {

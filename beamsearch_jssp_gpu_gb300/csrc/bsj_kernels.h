@@ -107,6 +107,7 @@ struct SearchCfg {
     unsigned long long* spill;  // candidate keys past list_cap (offsets as StepArgs::keys)
     int32_t cluster, lanes, rs, stage_stride;
     uint32_t c_magic;
+    uint32_t paths;             // kPath* bits of the launch itself
     int32_t list_cap, buf_cap;
     int32_t wide;               // report the cluster route
     int32_t ahead;              // the staging area holds a block's whole share

@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
         B.WL = (((d.n + 3) >> 2) + G - 1) / G;   // ready-position words per lane
         B.P = 1;
         B.parents = 0;
-        B.paths = 0;
+        B.paths = cf.paths;
         B.levels = 0;
         B.expanded = B.slots = B.mat = 0;
         B.beam0 = a.beam_pool + d.beam_off[0];
@@ -960,7 +960,9 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             B.parents = P;
             s_any = (int)slow;
             const bool large = V > kStageKeys || B.K > kLsdMax;
-            if (R > 0 && !lastlv) B.paths |= large ? kPathLarge : (cf.wide && C > 1 && V > kClusterMinKeys ? kPathCluster : kPathDirect);
+            if (R > 0 && !lastlv)
+                B.paths |= (large ? kPathLarge : (cf.wide && C > 1 && V > kClusterMinKeys ? kPathCluster : kPathDirect)) |
+                           (tries ? kPathRecount : 0u) | (tie ? kPathTieBins : 0u);
         }
         if (lastlv || keff == 0) break;    // clean: every child pruned
         if (!V1) bulk_wait();              // this level's children are in memory before barrier #2
@@ -1091,6 +1093,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                     }
                 } else {
                     sort_window(win + x0, buf, x1 - x0, x0, w0, w1, sel);
+                    if (tid == 0) B.paths |= kPathWindowSort;
                 }
             }
         } else if (R > 0) {
@@ -1099,6 +1102,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             // kernel's shared memory)
             const SegDesc& d = a.segs[seg];
             const int words = d.words;
+            if (tid == 0) B.paths |= kPathOneBlock;
             if (usemask)
 #pragma unroll 1
                 for (int i = tid; i < cnt * words; i += T) a.masks[d.mask_off + (int64_t)lo * words + i] = masks[i];
@@ -1280,8 +1284,8 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
         st.materialized += B.mat;
         st.levels += B.levels;
         st.P = B.P;
-        atomicOr(&st.select_paths, B.paths);
     }
+    if (tid == 0) atomicOr(&a.st[seg].select_paths, B.paths);
     csync();   // peers may read this block's counts until here
 }
 
@@ -1310,6 +1314,9 @@ bool search_layout(SearchCfg& cf, int cluster, int lanes, int kmax, int nmax, in
     const int words = (nmax + 31) / 32;
     cf.cluster = cluster;
     cf.lanes = lanes;
+    cf.paths = kPathResident;
+    for (int k = 0; k < (int)(sizeof(kSearchSizes) / sizeof(kSearchSizes[0])); k++)
+        if (kSearchSizes[k] == cluster) cf.paths |= 1u << (kPathBlocks + k);
     cf.c_magic = ((1u << 20) + (uint32_t)cluster - 1) / (uint32_t)cluster;   // x / cluster, x < 2^15
     cf.stage_stride = smax + ((smax >> 4) & 1 ? 0 : 16);   // odd in 16-byte units: groups' words on distinct banks
     for (cf.rs = T / lanes; cf.rs >= 16; cf.rs /= 2) {

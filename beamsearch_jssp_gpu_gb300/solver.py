@@ -225,12 +225,15 @@ class Plan:
         self.ctx._check(self.lib.bsj_plan_set_select_route(self.h, v))
 
     def set_select_cluster(self, on: bool):
-        """Cluster select where the rule picks it (True, the default) or one thread block per
-        beam (False) from the next run on (bsj_plan_set_select_cluster); results unchanged."""
+        """As many thread blocks per beam as the rule picks (True, the default) or the narrow forms
+        (False: 4 or 8 at most, one for the level kernels' selections) from the next run on
+        (bsj_plan_set_select_cluster); results unchanged."""
         self.ctx._check(self.lib.bsj_plan_set_select_cluster(self.h, 1 if on else 0))
 
     def select_routes(self) -> set:
-        """Names (``_native.ROUTE``) of the selection routes the last run took."""
+        """Names (``_native.ROUTE``) of the selection routes the last run took; "resident" and
+        the names after it tell what ran in the resident search, where "direct", "cluster" and
+        "large" only name its levels' size classes (bsj_plan_select_routes)."""
         r = ctypes.c_uint32()
         self.ctx._check(self.lib.bsj_plan_select_routes(self.h, ctypes.byref(r)))
         return {k for k, bit in nat.ROUTE.items() if r.value & bit}

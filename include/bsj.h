@@ -183,10 +183,18 @@ bsj_status bsj_plan_kernel_ms(const bsj_plan *plan, float *ms, int64_t *launches
    bsj_plan_select_routes: BSJ_ROUTE_* bits of the routes the last run took (OR over the
    plan's beams and levels; waits for the run).
    With no flags and no forced k_step form the gpu modes run the resident search (m >= 2):
-   one launch for all levels, 1 to 16 thread blocks per beam.  It reports a level's class:
-   LARGE for more than 16384 candidate keys or K > 8192, CLUSTER for more than 4096 keys
-   split over several blocks, DIRECT otherwise; levels whose tied scores exceed its buffers
-   run the one-block routes and report those too. */
+   one launch for all levels, 1 to 16 thread blocks per beam.  What ran there:
+     RESIDENT     some beam was searched by it;
+     BLOCKS(c)    with c = 1, 2, 4, 8, 12 or 16 thread blocks;
+     RECOUNT      a level's score bins were counted again over another range;
+     TIE_BINS     bins for tied scores (by makespan, noise value and slot range);
+     WINDOW_SORT  some block sorted its window (its bins too large to rank by counting);
+     ONE_BLOCK    a level's bins did not fit the blocks' buffers and one block selected it by the
+                  routes above, which are then reported too.
+   It also names each level's size class by three of the bits above -- the route the level
+   kernels would take, not code that ran: LARGE for more than 16384 candidate keys or K > 8192,
+   CLUSTER for more than 4096 keys in the default form with several blocks per beam, DIRECT
+   otherwise (in the narrow form also with several blocks). */
 #define BSJ_SELECT_FORCE_LARGE 1  /* large-level route (keys read in place) at any size */
 #define BSJ_SELECT_NO_LARGE    2  /* never the large-level route */
 #define BSJ_SELECT_NO_DIRECT   4  /* compact the survivors first (no direct staged pass) */
@@ -205,6 +213,13 @@ bsj_status bsj_plan_kernel_ms(const bsj_plan *plan, float *ms, int64_t *launches
 #define BSJ_ROUTE_RAW_LSD  64
 #define BSJ_ROUTE_BITONIC  128
 #define BSJ_ROUTE_CLUSTER  256
+#define BSJ_ROUTE_RESIDENT    512
+#define BSJ_ROUTE_RECOUNT     1024
+#define BSJ_ROUTE_TIE_BINS    2048
+#define BSJ_ROUTE_WINDOW_SORT 4096
+#define BSJ_ROUTE_ONE_BLOCK   8192
+#define BSJ_ROUTE_BLOCKS(c) /* c thread blocks per beam */ \
+    ((c) == 1 ? 1 << 16 : (c) == 2 ? 1 << 17 : (c) == 4 ? 1 << 18 : (c) == 8 ? 1 << 19 : (c) == 12 ? 1 << 20 : 1 << 21)
 bsj_status bsj_plan_set_select_route(bsj_plan *plan, int32_t flags);
 bsj_status bsj_plan_select_routes(bsj_plan *plan, uint32_t *routes);
 /* enable = 0: the narrow forms for this plan from its next run on, whatever K (a throughput
@@ -212,7 +227,8 @@ bsj_status bsj_plan_select_routes(bsj_plan *plan, uint32_t *routes);
    resident search with at most 4 thread blocks per beam (8 for wide beams of long lists,
    where they cost hardly more SM time), and one block per beam for the level kernels'
    selections; enable != 0 (the default): as wide as the rule picks.  Both forms' graphs are
-   kept, so switching costs one capture per form; the results never depend on it.  The route flags above take precedence. */
+   kept, so switching costs one capture per form; the results never depend on it.  The route
+   flags above take precedence. */
 bsj_status bsj_plan_set_select_cluster(bsj_plan *plan, int32_t enable);
 
 /* ---- Autotuning (no counterpart in the reference, whose launch shape is fixed:
