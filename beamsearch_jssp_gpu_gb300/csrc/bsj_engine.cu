@@ -84,8 +84,8 @@ struct bsj_plan {
     };
     std::vector<Group> groups;        // all beams, for the level kernels (forced forms and routes)
     std::vector<Group> rest_groups;   // the beams the resident search does not take
-    // resident search (bsj_search.cu): launches of [0] the rule's blocks per beam, [1] at most
-    // kSearchNarrow of them (bsj_plan_set_select_cluster)
+    // resident search (bsj_search.cu): launches of [0] the rule's blocks per beam, [1] the narrow
+    // form's (bsj_plan_set_select_cluster, search_shares)
     struct Search {
         SearchCfg cf{};
         int nbeams = 0;
@@ -121,7 +121,7 @@ struct bsj_plan {
     // launch; [2], [3] the same with the cluster select switched off
     cudaGraphExec_t graph[kNumStepVariants + 1][4] = {};
     bool select_cluster = true;   // bsj_plan_set_select_cluster: the cluster select where the rule picks it
-    bool cluster_matters = false; // some beam group is wide enough for the rule to pick it
+    bool cluster_matters = false; // the two forms differ
     int cluster_beams = 0;        // gpu-mode beams of K >= kSelectClusterMinK (their selects run at once)
     // timing
     bool timing = false;
@@ -319,9 +319,11 @@ double search_makespan(const std::vector<double>& us, const std::vector<int>& bl
 // Blocks per beam of the plan's resident searches: for each largest size, every beam at its
 // fastest, or only as wide as finishing within 1, 1.5, 2 or 3 times the longest search needs;
 // the choice with the smallest estimated makespan.  (Few beams end up wide, a batch's short
-// searches narrow.)
-std::vector<int> search_shares(const bsj_plan* p, int cmax_form)
+// searches narrow.)  With `rule`, the default form's choice, the narrow form: sizes up to
+// kSearchNarrow, 8 for wide beams of long lists, and no beam wider than by the rule.
+std::vector<int> search_shares(const bsj_plan* p, const std::vector<int>* rule)
 {
+    const int cmax_form = rule ? kSearchNarrow : kSearchMaxCluster;
     const SearchDevice& dev = p->ctx->search;
     const int count = p->nseg - p->nrest;
     constexpr int kSizes = sizeof(kSearchSizes) / sizeof(kSearchSizes[0]);
@@ -359,13 +361,15 @@ std::vector<int> search_shares(const bsj_plan* p, int cmax_form)
     }
     // the narrow form saves SM time, and wide beams of long lists spend hardly more of it on
     // eight blocks (100x15 K=4 096, estimated: 4 x 53.9 or 8 x 27.8 us per level)
-    if (cmax_form == kSearchNarrow && dev.clusters[8] > 0)
+    if (rule)
         for (int i = 0; i < count; i++) {
             const SegDesc& d = p->segs[p->nrest + i];
             const bool v1 = d.mode == BSJ_MODE_V1;
-            if (search_blocks(dev, d.n, d.m, d.K, v1, 8) == 8 &&
+            if (dev.clusters[8] > 0 && search_blocks(dev, d.n, d.m, d.K, v1, 8) == 8 &&
                 8 * search_level_us(d.n, d.K, v1, 8) <= 1.1 * best[i] * search_level_us(d.n, d.K, v1, best[i]))
                 best[i] = 8;
+            // (140 beams of 100 jobs, K=4096, have one block each by the rule)
+            best[i] = std::min(best[i], (*rule)[i]);
         }
     return best;
 }
@@ -375,10 +379,12 @@ std::vector<int> search_shares(const bsj_plan* p, int cmax_form)
 void plan_searches(bsj_plan* p, std::vector<int32_t>& list, int32_t* d_list, unsigned long long* spill)
 {
     const SearchDevice& dev = p->ctx->search;
+    const std::vector<int> rule = search_shares(p, nullptr), narrow = search_shares(p, &rule);
+    p->cluster_matters = narrow != rule;
     for (int form = 0; form < 2; form++) {
         struct Class { int c, lanes, kmax, nmax, opsmax, smax; bool v1; double us; std::vector<int32_t> segs; };
         std::vector<Class> classes;
-        const std::vector<int> share = search_shares(p, form == 0 ? kSearchMaxCluster : kSearchNarrow);
+        const std::vector<int>& share = form == 0 ? rule : narrow;
         for (int si = p->nrest; si < p->nseg; si++) {
             const SegDesc& d = p->segs[si];
             const int S = SearchLay(d.n, d.m).bytes, c = share[si - p->nrest], lanes = search_lanes(d.n, d.K, c);
@@ -418,7 +424,7 @@ void plan_searches(bsj_plan* p, std::vector<int32_t>& list, int32_t* d_list, uns
             search_layout(sr.cf, x.c, x.lanes, x.kmax, x.nmax, x.opsmax, x.smax, dev.smem);
             sr.cf.list = d_list + at;
             sr.cf.spill = spill;
-            sr.cf.wide = form == 0 ? 1 : 0;
+            sr.cf.wide = form == 0 || !p->cluster_matters ? 1 : 0;
             sr.nbeams = (int)x.segs.size();
             sr.v1 = x.v1;
             for (int32_t si : x.segs) list[at++] = si;
@@ -769,11 +775,9 @@ bsj_status plan_build(bsj_context* ctx, int ninst, const bsj_instance* insts, in
     if (p->nrest > 0) make_groups(0, p->nrest, p->rest_groups);
     for (const SegDesc& d : p->segs)
         if (d.mode <= BSJ_MODE_CLEAN && d.K >= kSelectClusterMinK) p->cluster_beams++;
-    // the select form differs where the resident search gives some beam several blocks, or the
+    // the select form differs where the resident search gives some beam other blocks, or the
     // level kernels' cluster select applies (too many wide beams for even 2 CTAs each: not)
-    p->cluster_matters = p->cluster_beams > 0 && (int64_t)p->cluster_beams * 2 <= ctx->sm_count;
-    for (const auto& sr : p->search[0])
-        if (sr.cf.cluster > kSearchNarrow) p->cluster_matters = true;
+    if (p->cluster_beams > 0 && (int64_t)p->cluster_beams * 2 <= ctx->sm_count) p->cluster_matters = true;
     cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming);
     for (cudaEvent_t& ev : p->join) cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
     // chunk sizes: the default rule per group; the variant tuning found for this shape on

@@ -69,7 +69,7 @@ constexpr int kSearchThreads = 512;
 constexpr int kSearchBinBits = 9;
 constexpr int kSearchBins = 1 << kSearchBinBits;   // score bins of the selection
 constexpr int kSearchMaxCluster = 16;
-constexpr int kSearchNarrow = 4;       // blocks per beam at most with the cluster forms switched off
+constexpr int kSearchNarrow = 4;       // blocks per beam of the narrow form, but for search_shares' 8
 constexpr int kSearchMinBuf = 2048;    // keys the sort's buffer holds at least
 constexpr int kSearchMinList = 1024;   // candidate keys the list holds at least
 
@@ -127,7 +127,7 @@ cudaError_t search_device(SearchDevice& out);
 // Estimated microseconds per level with C blocks (for choosing C only).
 double search_level_us(int n, int K, bool v1, int C);
 // Blocks per beam with the smallest estimate among sizes up to cmax that the device runs and
-// whose layout fits; 0 if there is none.
+// whose layout fits, or the smallest size above where there is none; 0 if nothing fits.
 int search_blocks(const SearchDevice& dev, int n, int m, int K, bool v1, int cmax);
 // Lanes per survivor for C blocks.
 int search_lanes(int n, int K, int C);

@@ -26,3 +26,21 @@ def test_narrow_form_matches_oracle(ctx, beams):
         for f in ("makespan", "found", "expanded", "slots", "levels"):
             assert got[i][f] == want[f], (f, beams[i])
         assert np.array_equal(got[i]["seq"], want["seq"]), beams[i]
+
+
+@pytest.mark.parametrize("first", [True, False])
+def test_narrow_form_is_no_wider(ctx, first):
+    # so many beams that the rule gives each one block: the narrow form, which trades latency for
+    # SM time, gives them no more, and the form asked for first does not stand in for the other
+    inst = [synthetic_instance(100, 2, 1)]
+    want = O.solve(*inst[0], "v2", 4096, 3)
+    plan = ctx.plan(inst, [BeamSpec("v2", 4096, 500000, i, 0, -1) for i in range(140)])
+    try:
+        for wide in (first, not first):
+            plan.set_select_cluster(wide)
+            plan.run()
+            got = plan.results()
+            assert {r for r in plan.select_routes() if r.startswith("blocks")} == {"blocks_1"}, wide
+            assert got[3]["makespan"] == want["makespan"] and np.array_equal(got[3]["seq"], want["seq"]), wide
+    finally:
+        plan.close()
