@@ -375,9 +375,11 @@ std::vector<int> search_shares(const bsj_plan* p, const std::vector<int>* rule)
 }
 
 // The plan's resident-search launches: beams sharing a block count, lane count and mode
-// class run in one launch, longest search first.
-void plan_searches(bsj_plan* p, std::vector<int32_t>& list, int32_t* d_list, unsigned long long* spill)
+// class run in one launch, longest search first.  `list` receives the launches' beams; true if
+// some block's candidate list may outgrow its shared memory (the plan then holds a spill region).
+bool plan_searches(bsj_plan* p, std::vector<int32_t>& list)
 {
+    bool spills = false;
     const SearchDevice& dev = p->ctx->search;
     const std::vector<int> rule = search_shares(p, nullptr), narrow = search_shares(p, &rule);
     p->cluster_matters = narrow != rule;
@@ -422,15 +424,18 @@ void plan_searches(bsj_plan* p, std::vector<int32_t>& list, int32_t* d_list, uns
             std::stable_sort(x.segs.begin(), x.segs.end(), [&](int32_t a, int32_t b) { return us(a) > us(b); });
             bsj_plan::Search sr;
             search_layout(sr.cf, x.c, x.lanes, x.kmax, x.nmax, x.opsmax, x.smax, dev.smem);
-            sr.cf.list = d_list + at;
-            sr.cf.spill = spill;
             sr.cf.wide = form == 0 || !p->cluster_matters ? 1 : 0;
             sr.nbeams = (int)x.segs.size();
             sr.v1 = x.v1;
-            for (int32_t si : x.segs) list[at++] = si;
+            for (int32_t si : x.segs) {
+                const SegDesc& d = p->segs[si];
+                if ((int64_t)((d.K + x.c - 1) / x.c) * d.n > sr.cf.list_cap) spills = true;
+                list[at++] = si;
+            }
             p->search[form].push_back(sr);
         }
     }
+    return spills;
 }
 
 // With `bytes_only` non-null, computes the plan's device footprint into it and allocates
@@ -605,6 +610,9 @@ bsj_status plan_build(bsj_context* ctx, int ninst, const bsj_instance* insts, in
         return fail(ctx, BSJ_ERR_LIMIT, "beam too wide for the shared-memory select");
     }
 
+    std::vector<int32_t> slist(2 * (size_t)nbeams, 0);
+    const bool spills = plan_searches(p, slist);
+
     // device memory layout (one allocation)
     size_t o = 0;
     auto take = [&](size_t bytes) { size_t at = o; o = align_up(o + bytes, 256); return at; };
@@ -621,7 +629,7 @@ bsj_status plan_build(bsj_context* ctx, int ninst, const bsj_instance* insts, in
     const size_t o_beam = take(off_beam);
     const size_t o_slot = take(off_slot);
     const size_t o_keys = take(8 * off_keys);
-    const size_t o_spill = take(p->nrest < nbeams ? 8 * off_keys : 0);
+    const size_t o_spill = take(spills ? 8 * off_keys : 0);
     const size_t o_slist = take(2 * sizeof(int32_t) * nbeams);
     const size_t o_sel = take(4 * off_sel);
     const size_t o_mask = take(4 * off_mask);
@@ -681,9 +689,14 @@ bsj_status plan_build(bsj_context* ctx, int ninst, const bsj_instance* insts, in
     a.noise = reinterpret_cast<const float*>(base + o_noise);
     a.dnoise = reinterpret_cast<const double*>(base + o_dnoise);
 
-    std::vector<int32_t> slist(2 * (size_t)nbeams, 0);
-    plan_searches(p, slist, reinterpret_cast<int32_t*>(base + o_slist),
-                  reinterpret_cast<unsigned long long*>(base + o_spill));
+    for (int form = 0; form < 2; form++) {
+        const int32_t* at = reinterpret_cast<const int32_t*>(base + o_slist) + (size_t)form * nbeams;
+        for (auto& sr : p->search[form]) {
+            sr.cf.list = at;
+            sr.cf.spill = spills ? reinterpret_cast<unsigned long long*>(base + o_spill) : nullptr;
+            at += sr.nbeams;
+        }
+    }
 
     // uploads (synchronous: the host vectors are pageable)
     cudaStream_t st = ctx->stream;

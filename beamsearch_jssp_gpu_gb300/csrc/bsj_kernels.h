@@ -104,7 +104,7 @@ __host__ __device__ __forceinline__ bool search_position_ok(int i, uint32_t head
 // One launch: its beams, blocks per beam, lanes per survivor and shared-memory layout.
 struct SearchCfg {
     const int32_t* list;        // the launch's beams
-    unsigned long long* spill;  // candidate keys past list_cap (offsets as StepArgs::keys)
+    unsigned long long* spill;  // candidate keys past list_cap (offsets as StepArgs::keys; null: lists fit)
     int32_t cluster, lanes, rs, stage_stride;
     uint32_t c_magic;
     uint32_t paths;             // kPath* bits of the launch itself

@@ -1342,7 +1342,7 @@ bool search_layout(SearchCfg& cf, int cluster, int lanes, int kmax, int nmax, in
         cf.ahead = pc > cf.rs && pc <= kMaxAhead * cf.rs && o + whole + std::min(want, (size_t)pc * 48) <= limit ? 1 : 0;
         if (cf.ahead) stage = std::max(stage, whole);
         if (o + stage + (size_t)kSearchMinList * 8 > limit) continue;
-        const size_t lst = std::min(want, limit - o - stage) & ~(size_t)15;
+        const size_t lst = std::min((want + 15) & ~(size_t)15, (limit - o - stage) & ~(size_t)15);
         cf.list_cap = (int)(lst / 8);
         cf.off_list = take(lst);
         cf.off_stage = (int)o;
