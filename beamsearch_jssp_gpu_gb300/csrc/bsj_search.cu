@@ -892,7 +892,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                 break;
             }
             // ---- again, over the range from the level's lowest score to the bin of the last
-            // survivor: linear bins, then (or at once, if the last level had them) tie bins
+            // survivor: linear bins, then (at once, if the level had them or has one try only) tie bins
             tries++;
             uint32_t mn = 0xFFFFFFFFu, mx = 0u;
 #pragma unroll 1
@@ -929,7 +929,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             const bool was = tie;
             if (!was && Tb < NB - 1)
                 mx = (uint32_t)min((unsigned long long)mx, plo + ((unsigned long long)(Tb + 1) << shift) - 1);
-            if (was || tries > 1) {
+            if (was || tries > 1 || !recount_ok) {
                 const float ns = (float)(t + 1), per = __fdiv_rn(ns, (float)B.unit);
                 const int c0 = __float2int_rn(__uint_as_float(mn) * per);
                 int c1 = __float2int_rn(__uint_as_float(mx) * per);
@@ -1102,7 +1102,10 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             // kernel's shared memory)
             const SegDesc& d = a.segs[seg];
             const int words = d.words;
-            if (tid == 0) B.paths |= kPathOneBlock;
+            if (tid == 0) {
+                B.paths |= kPathOneBlock;
+                s_any = 1;   // tie bins next: a level of linear bins that went here would repeat itself
+            }
             if (usemask)
 #pragma unroll 1
                 for (int i = tid; i < cnt * words; i += T) a.masks[d.mask_off + (int64_t)lo * words + i] = masks[i];

@@ -52,3 +52,12 @@ def test_tied_levels_stay_resident(ctx, name, n, m, K):
     mc, du = synthetic_instance(n, m, 4)
     _, routes = _solve(ctx, mc, DURATIONS[name](du).astype(np.int32), "v2", K, 500000)
     assert not routes & {"bucket", "radix"}, routes
+
+
+@pytest.mark.parametrize("mode,n,m", [("v2", 20, 3), ("clean", 30, 3), ("v1", 24, 4)])
+def test_wide_tied_levels_leave_one_block(ctx, mode, n, m):
+    # a wide beam whose early levels fit no bins goes on with tie bins: it does not stay with one block
+    # (v1's stale slots bring back equal states in neighbouring ranks, which no bin tells apart)
+    mc, du = synthetic_instance(n, m, n + m)
+    _, routes = _solve(ctx, mc, DURATIONS["small"](du).astype(np.int32), mode, 16384, 500000)
+    assert "tie_bins" in routes and (mode == "v1" or "one_block" not in routes), routes
