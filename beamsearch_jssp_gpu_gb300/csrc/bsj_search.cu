@@ -332,6 +332,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
     __shared__ int s_T, s_first, s_maxbin, s_x0, s_x1, s_mymax, s_valid, s_lcount, s_tie;
     __shared__ int s_slow;             // ranking the last level with linear bins was slow
     __shared__ uint4 s_lin;            // score bins: plo, shift, tie; levels left with tie bins | the last stay << 16
+    __shared__ int s_bad;              // a survivor entry or position that names nothing
     __shared__ int s_any;              // s_slow of some block
 
     int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -401,6 +402,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
         s_valid = 0;
         s_lcount = 0;
         s_slow = 0;
+        s_bad = 0;
         s_lin = make_uint4(0u, 21u, 0u, 1u << 16);
     }
     load_tables();
@@ -504,14 +506,11 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             uint8_t* const mcb = sb + B.off_mc;
             uint4* const hdr = reinterpret_cast<uint4*>(sb + B.off_hdr);   // r | ns << 16, cmax, lineage, stamp
             if (t > 0) {
-                if (act) {
-                    e = sel[rl];
-                    if (!search_entry_ok(e, B.parents, n)) {
-                        // no survivor: it takes no part
-                        if (gl == 0) atomicOr(&a.st[seg].status, kStatusBadSelect);
-                        act = false;
-                    }
-                }
+                // (an entry that is no survivor takes no part)
+                if (act) e = sel[rl];
+                const bool entry = search_entry_ok(e, B.parents, n);
+                if (act && !entry) s_bad = 1;
+                act = act && entry;
                 if (V1) {
                     if (act) {
                         const int c = (int)((e & ~kFillerFlag) >> 7);
@@ -544,7 +543,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                         phase ^= 1u << k;
                         if (!ok) {
                             // a copy that never completed: its survivors take no further part
-                            if (lane == 0) atomicOr(&a.st[seg].status, kStatusBadSelect);
+                            if (lane == 0) s_bad = 1;
                             act = false;
                         }
                     }
@@ -634,7 +633,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                         for (int q = gl; q < (S >> 4); q += G) reinterpret_cast<uint4*>(sb)[q] = __ldcg(s4 + q);
                         if (gl == 0) {
                             B.hist[(t - 1) * B.K + r] = kMark;
-                            if (B.mode == MODE_CLEAN || !(e & kFillerFlag)) atomicOr(&a.st[seg].status, kStatusBadSelect);
+                            if (B.mode == MODE_CLEAN || !(e & kFillerFlag)) s_bad = 1;
                         }
                     }
                     __syncwarp();
@@ -1288,7 +1287,10 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
         st.levels += B.levels;
         st.P = B.P;
     }
-    if (tid == 0) atomicOr(&a.st[seg].select_paths, B.paths);
+    if (tid == 0) {
+        atomicOr(&a.st[seg].select_paths, B.paths);
+        if (s_bad) atomicOr(&a.st[seg].status, kStatusBadSelect);
+    }
     csync();   // peers may read this block's counts until here
 }
 
