@@ -1346,6 +1346,10 @@ bool search_layout(SearchCfg& cf, int cluster, int lanes, int kmax, int nmax, in
         const size_t whole = (size_t)pc * cf.stage_stride;
         cf.ahead = pc > cf.rs && pc <= kMaxAhead * cf.rs && o + whole + std::min(want, (size_t)pc * 48) <= limit ? 1 : 0;
         if (cf.ahead) stage = std::max(stage, whole);
+        // wide shares: the largest buffer where a third more makes it (a bin too large for the buffer
+        // sends the level to one block).  v1 100x8 K=16384: 577 -> 354 us per level
+        const size_t most = (size_t)kSortMax * 12;
+        if (pc >= 512 && stage < most && most - stage <= stage / 3 && o + most + (size_t)pc * 48 <= limit) stage = most;
         if (o + stage + (size_t)kSearchMinList * 8 > limit) continue;
         const size_t lst = std::min((want + 15) & ~(size_t)15, (limit - o - stage) & ~(size_t)15);
         cf.list_cap = (int)(lst / 8);
