@@ -290,6 +290,30 @@ int rule_chunk_var(int64_t ranks, int nq, int64_t granks, bool group_ok, int kma
     return chunk_var_of((nq == 4 || granks > 8192) ? 32 : 16);
 }
 
+// v1 beams that the level kernels search faster.  In the resident search a beam's 16 SMs write every
+// scored child's snapshot (~30 bytes per cycle and SM), and a share of several rounds copies its
+// survivors twice; the level kernels write from all SMs.  `children`: what a level scores, a
+// survivor having 1 + (n - 1) / m candidates.  GB300, us per level, durations U[1, 99], level kernels |
+// resident:
+//   n <= 32: the resident search always (24x4 K=4096: 37 | 31, K=6144: 95 | 45).
+//   K <= 2048, and K < 4096 below 65 jobs, where a share is one round: 64x5 K=2560: 61 | 46.  Above, two
+//   rounds: 128x4 K=2560: 108 | 126, 128x8: 74 | 88, 80x2: 106 | 131; but 80x8: 59 | 49, 100x5: 81 | 80.
+//   From 4096 on the level kernels select up to 65 536 children in shared memory: 64x5 K=4096: 44 | 67,
+//   50x5 K=6144: 56 | 82, 40x8 K=5120: 44 | 59, 128x15 K=6144: 87 | 142; above 65 536, 64x3 K=4096:
+//   101 | 83, 50x4 K=5120: 111 | 79.  At 4096 a share is one round up to 64 jobs, and it takes 11 MB of
+//   children: 64x10 (15 MB): 38 | 42, 50x8 (12 MB): 37 | 39, 50x10 (10 MB): 37 | 34.
+//   From 8192 on their selection takes 100-400 us: 40x4: 294 | 99, 128x10: 216 | 192.  (128x5, 80x2
+//   and their like lose there too, 286 | 342 at K=8192, but with tied scores win: 485 | 356.)
+bool v1_level_kernels(int n, int m, int K)
+{
+    if (n <= 32 || K <= 2048 || K >= 8192) return false;
+    const double children = K * (1.0 + (n - 1.0) / m);
+    if (K < kSelectClusterMinK) return n > 110 || (n > 64 && m == 2);
+    if (children > 66500) return false;   // (an estimate: most levels have fewer)
+    if (K > kSelectClusterMinK) return true;
+    return n > 64 ? n > 90 : children * SearchLay(n, m).bytes > 11e6;
+}
+
 // Estimated makespan (us) of the resident searches with blocks[i] blocks each, started
 // longest first as the device's SMs allow.
 double search_makespan(const std::vector<double>& us, const std::vector<int>& blocks, int sms)
@@ -495,6 +519,7 @@ bsj_status plan_build(bsj_context* ctx, int ninst, const bsj_instance* insts, in
         const int i = beams[b].instance;
         return beams[b].mode >= BSJ_MODE_V1 && beams[b].mode <= BSJ_MODE_CLEAN && i >= 0 && i < ninst &&
                insts[i].m >= 2 && beams[b].beam_width >= 1 && beams[b].beam_width <= BSJ_MAX_BEAM &&
+               !(beams[b].mode == BSJ_MODE_V1 && v1_level_kernels(insts[i].n, insts[i].m, beams[b].beam_width)) &&
                search_blocks(ctx->search, insts[i].n, insts[i].m, beams[b].beam_width,
                              beams[b].mode == BSJ_MODE_V1, kSearchMaxCluster) > 0;
     };

@@ -68,3 +68,14 @@ def test_one_block_levels(ctx, mode, n, m, K, dmax, wide):
 def test_plain_levels_take_no_detour(ctx):
     got = _routes(ctx, [BeamSpec("v2", 256, 500000, 3, 0, -1)], [synthetic_instance(15, 15, 1)])
     assert not got & {"one_block", "bucket", "radix", "large"}, got
+
+
+@pytest.mark.parametrize("n,m,K,resident", [
+    (32, 4, 5000, True), (40, 8, 5120, False), (40, 3, 5120, True), (50, 5, 4096, False), (50, 10, 4096, True),
+    (64, 6, 8191, True), (64, 8, 7000, False), (64, 6, 8192, True), (80, 2, 2560, False), (80, 5, 2560, True),
+    (128, 2, 2048, True), (128, 3, 2049, False), (100, 9, 4096, False), (100, 8, 6144, True)])
+def test_v1_beams_by_size(ctx, n, m, K, resident):
+    # v1 writes every scored child: beams of many children go to the level kernels (v2 and clean never)
+    inst = synthetic_instance(n, m, 2)
+    got = _routes(ctx, [BeamSpec("v1", K, 500000, 3, 0, -1)], [inst])
+    assert ("resident" in got) == resident, got
