@@ -333,7 +333,6 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
     __shared__ int s_slow;             // ranking the last level with linear bins was slow
     __shared__ uint4 s_lin;            // score bins: plo, shift, tie; levels left with tie bins | the last stay << 16
     __shared__ int s_bad;              // a survivor entry or position that names nothing
-    __shared__ int s_any;              // s_slow of some block
 
     int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int C = cf.cluster;
@@ -957,7 +956,6 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             B.mat += lastlv ? 0 : keff;
             B.P = keff;
             B.parents = P;
-            s_any = (int)slow;
             const bool large = V > kStageKeys || B.K > kLsdMax;
             if (R > 0 && !lastlv)
                 B.paths |= (large ? kPathLarge : (cf.wide && C > 1 && V > kClusterMinKeys ? kPathCluster : kPathDirect)) |
@@ -966,6 +964,46 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
         if (lastlv || keff == 0) break;    // clean: every child pruned
         if (!V1) bulk_wait();              // this level's children are in memory before barrier #2
         const bool fits = R == 0 || (H < 0xFFFF && Pn + 2 * H <= cf.buf_cap);
+        // ---- the next level's bins: this level's kept scores, one operation later (in a warp that has
+        // no keys to push where the share is small)
+        if (tid == T - 32 && R == 0) s_lin.z = 0u;
+        if (tid == T - 32 && R > 0) {
+            const uint4 lin = s_lin;
+            // linear bins did not do: some block ranked the last level slowly, or this one goes to one block
+            const bool failed = slow != 0u || !fits;
+            const float u = __fdividef(1.0f, (float)(t + 2));
+            // f0, f1: the scores kept.  The lowest child keeps its makespan; above, half the kept range
+            // and some more (a narrow beam's range is a few operations' differences wide, and a
+            // prediction that misses it clamps all keys into one bin)
+            float f0 = __uint_as_float(lin.x + ((uint32_t)s_first << lin.y));
+            float f1 = __uint_as_float(lin.x + (((uint32_t)Tb + 1u) << lin.y) - 1u);
+            int left = (int)(lin.w & 0xFFFFu), stay = (int)(lin.w >> 16), next_tie = 0;
+            if (lin.z | (uint32_t)failed | (lin.w ^ (1u << 16))) {
+                // tie bins for the next levels where linear ones did not do, and for twice as many
+                // each time that they do not again
+                if (lin.z) {
+                    const TieMap& m = s_tm[tm];
+                    const float score = __fdiv_rn((float)m.unit, m.ns);
+                    f0 = (float)(m.c0 + min(s_first / m.q, m.nc)) * score;
+                    f1 = (float)(m.c0 + min(Tb / m.q, m.nc) + 1) * score;
+                }
+                if (left > 0) left--;
+                else if (lin.z || failed) left = stay = min(2 * stay, kTieStay);
+                else stay = max(stay / 2, 1);
+                if (left > 0) {
+                    const float g0 = f0 - f0 * u, g1 = f1 + 0.5f * (f1 - f0) + B.slack * u;
+                    const float ns = (float)(t + 2), per = __fdiv_rn(ns, (float)B.unit);
+                    const int c0 = __float2int_rn(g0 * per), c1 = __float2int_rn(g1 * per);
+                    next_tie = (uint32_t)(c1 - c0) < (uint32_t)NB ? 1 : 0;
+                    if (next_tie) tie_map(s_tm[tm ^ 1], c0, c1 - c0 + 1, B.unit, ns, g0, keff);
+                }
+            }
+            const float g0 = f0 - f0 * u, g1 = f1 + 0.5f * (f1 - f0) + B.slack * u;
+            const uint32_t lo32 = __float_as_uint(g0), hi32 = __float_as_uint(g1);
+            const int nbits = hi32 > lo32 ? 32 - __clz(hi32 - lo32) : 0;
+            s_lin = make_uint4(lo32, (uint32_t)(nbits > kSearchBinBits ? nbits - kSearchBinBits : 0),
+                               (uint32_t)next_tie, (uint32_t)(left | stay << 16));
+        }
         if (R > 0 && fits) {
             // ---- keys of bins <= T to their positions' owners; buf[p - first position + H]
 #pragma unroll 1
@@ -1101,10 +1139,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             // kernel's shared memory)
             const SegDesc& d = a.segs[seg];
             const int words = d.words;
-            if (tid == 0) {
-                B.paths |= kPathOneBlock;
-                s_any = 1;   // tie bins next: a level of linear bins that went here would repeat itself
-            }
+            if (tid == 0) B.paths |= kPathOneBlock;
             if (usemask)
 #pragma unroll 1
                 for (int i = tid; i < cnt * words; i += T) a.masks[d.mask_off + (int64_t)lo * words + i] = masks[i];
@@ -1197,44 +1232,6 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                 for (int i = tid; i < cnt * d2.words; i += T)
                     masks[i] = __ldcg(a.masks + d2.mask_off + (int64_t)lo * d2.words + i);
             __syncthreads();
-        }
-        // ---- the next level's bins: this level's kept scores, one operation later (in a warp that has
-        // no keys to rank where the share is small)
-        if (tid == T - 32 && R == 0) s_lin.z = 0u;
-        if (tid == T - 32 && R > 0) {
-            const uint4 lin = s_lin;
-            const float u = __fdividef(1.0f, (float)(t + 2));
-            // f0, f1: the scores kept.  The lowest child keeps its makespan; above, half the kept range
-            // and some more (a narrow beam's range is a few operations' differences wide, and a
-            // prediction that misses it clamps all keys into one bin)
-            float f0 = __uint_as_float(lin.x + ((uint32_t)s_first << lin.y));
-            float f1 = __uint_as_float(lin.x + (((uint32_t)Tb + 1u) << lin.y) - 1u);
-            int left = (int)(lin.w & 0xFFFFu), stay = (int)(lin.w >> 16), next_tie = 0;
-            if (lin.z | (uint32_t)s_any | (lin.w ^ (1u << 16))) {
-                // tie bins for the next levels where linear ones did not do, and for twice as many
-                // each time that they do not again
-                if (lin.z) {
-                    const TieMap& m = s_tm[tm];
-                    const float score = __fdiv_rn((float)m.unit, m.ns);
-                    f0 = (float)(m.c0 + min(s_first / m.q, m.nc)) * score;
-                    f1 = (float)(m.c0 + min(Tb / m.q, m.nc) + 1) * score;
-                }
-                if (left > 0) left--;
-                else if (lin.z || s_any) left = stay = min(2 * stay, kTieStay);
-                else stay = max(stay / 2, 1);
-                if (left > 0) {
-                    const float g0 = f0 - f0 * u, g1 = f1 + 0.5f * (f1 - f0) + B.slack * u;
-                    const float ns = (float)(t + 2), per = __fdiv_rn(ns, (float)B.unit);
-                    const int c0 = __float2int_rn(g0 * per), c1 = __float2int_rn(g1 * per);
-                    next_tie = (uint32_t)(c1 - c0) < (uint32_t)NB ? 1 : 0;
-                    if (next_tie) tie_map(s_tm[tm ^ 1], c0, c1 - c0 + 1, B.unit, ns, g0, keff);
-                }
-            }
-            const float g0 = f0 - f0 * u, g1 = f1 + 0.5f * (f1 - f0) + B.slack * u;
-            const uint32_t lo32 = __float_as_uint(g0), hi32 = __float_as_uint(g1);
-            const int nbits = hi32 > lo32 ? 32 - __clz(hi32 - lo32) : 0;
-            s_lin = make_uint4(lo32, (uint32_t)(nbits > kSearchBinBits ? nbits - kSearchBinBits : 0),
-                               (uint32_t)next_tie, (uint32_t)(left | stay << 16));
         }
         if (keff > R) {
             // ---- v1 / v2: the lowest-numbered unscored slots follow, in slot order
