@@ -1,15 +1,20 @@
 // bsj_engine.cu -- host engine and the C ABI (include/bsj.h).
 //
 // A plan is a set of beams (independent seeds and/or instances of uneven size, any mix
-// of modes) laid out in one device allocation.  Running a plan enqueues every search level:
+// of modes) laid out in one device allocation.  Running a plan enqueues, on parallel branches:
+//
+//   k_search                                     all levels of a class of gpu-mode beams
+//
+// for the beams the resident search takes, and for the others (ICH, PMS, one machine; all beams
+// where a k_step form or a selection route is forced), per beam group:
 //
 //   k_step(-1)                                   roots + level-0 expansion
 //   for s = 0 .. maxN-1:
 //       k_select(s) / k_heap(s)                  top-K per beam (gpu modes / ICH, PMS)
 //       k_gather_v1(s)                           v1 beams only
 //       k_step(s)            (s < maxN-1)        materialise level s+1, expand it
-//   k_finalize                                   makespans + schedules
 //
+// then k_lineage and k_finalize (makespans + schedules),
 // replacing the reference's per-call host loop of three launches per level with device
 // memory allocated once per call (gpu/v1/solver.cu:178-298, gpu/v2_twophases/solver.cu:
 // 256-386).  The whole sequence is captured once into a CUDA graph and replayed.
@@ -752,8 +757,9 @@ bsj_status plan_build(bsj_context* ctx, int ninst, const bsj_instance* insts, in
     }
     int want = (p->total_ranks + kWarpsPerStepCta - 1) / kWarpsPerStepCta;
     p->gather_grid = std::max(1, std::min(want, ctx->sm_count * 8));
-    // beam groups, balanced by work (K * levels); BSJ_MAX_BEAM_GROUPS in the environment
-    // lowers the number of concurrent groups (1 = all beams in lockstep, for measurements)
+    // beam groups of the level kernels, balanced by work (K * levels); BSJ_MAX_BEAM_GROUPS in the
+    // environment lowers the number of concurrent groups (1 = all their beams in lockstep, for
+    // measurements; the resident searches are not touched)
     auto make_groups = [&](int first, int end, std::vector<bsj_plan::Group>& out_groups) {
         int gmax = kMaxBranches;
         if (const char* env = std::getenv("BSJ_MAX_BEAM_GROUPS")) {

@@ -40,9 +40,9 @@
 // threads: 1 024 measured 9.8 against 8.1 us per level at 15x15 K=256 (barriers and issue
 // slots), 256 12.0.  Snapshots by bulk copies: 256 of 448 bytes load in 2 350 cycles, by
 // 16-byte cp.async in 4 280.  GB300, us per call, level kernels -> this: 15x15 K=256 3 332 ->
-// 1 456; v1 20x15 K=1024 6 836 -> 2 932; v1 20x15 K=16384 64 083-75 838 -> 22 000-23 400;
-// 50x20 K=4096 24 288 -> 12 425, 8 beams 28 182 -> 16 042; 100x20 K=4096 8 beams 66 166 ->
-// 39 875.
+// 1 530; v1 20x15 K=1024 6 836 -> 2 950; v1 20x15 K=16384 64 083-75 838 -> 22 300;
+// 50x20 K=4096 24 288 -> 12 410, 8 beams 28 182 -> 16 050; 100x20 K=4096 8 beams 66 166 ->
+// 40 300.
 #include <algorithm>
 #include <mutex>
 #include <type_traits>
@@ -194,7 +194,7 @@ constexpr int kPlainBinMax = 96;
 // groups of equal scores up to kTieMax keys are ranked by counting, larger ones sorted with the
 // whole window.  256: 14.0 | 35.2 for the last two; 512: 13.9 | 35.2; 1 024: 13.9 | 34.6.
 constexpr int kTieMax = 1024;
-// a bin larger than kRecountBin: the level is counted again over its exact score range, which costs
+// a bin larger than kRecountBin: the level is counted again over a closer score range, which costs
 // a pass over the keys and two barriers.  384: 14.0 at 50x20 K=4096; 768 and 1 536: 13.5.
 constexpr int kRecountBin = 1536;
 constexpr int kMaxRecounts = 3;
@@ -1200,7 +1200,8 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
             // Nothing but the warps' copy phases stays in registers across the call: what does is
             // kept in local memory for the whole level loop (84-168 bytes per thread).  us per call
             // with and without: 15x15 K=256 1 654 -> 1 456, v1 20x15 K=1024 3 266 -> 2 932, 50x20
-            // K=4096 13 602 -> 12 425, 8 beams 17 539 -> 16 042, 100x20 8 beams 43 166 -> 39 875.
+            // K=4096 13 602 -> 12 425, 8 beams 17 539 -> 16 042, 100x20 8 beams 43 166 -> 39 875 (figures
+            // of the build that took them out).
             if (tid == 0)
                 s_keep = LevelState{seg, t, recount_ok ? 1 : 0, tm, lo, cnt, V, Vb, keff, R,
                                     Pn, w0, w1, Tb};
@@ -1339,7 +1340,9 @@ bool search_layout(SearchCfg& cf, int cluster, int lanes, int kmax, int nmax, in
         while (roomy < (size_t)pc + 4096) roomy *= 2;
         if (o + roomy * 12 + std::min(want, (size_t)pc * 128) <= limit) stage = std::max(stage, roomy * 12);
         // the whole share staged at once (2 to kMaxAhead rounds of it) where that leaves the
-        // list 6 keys per survivor (the levels of 50x20 hold 3.7)
+        // list 6 keys per survivor (the levels of 50x20 hold 3.7; fitted there -- lists of few machines
+        // hold more, 20 at 60x3, and keep part of them in L2: 60x3 K=4096 is faster than by the level
+        // kernels all the same)
         const size_t whole = (size_t)pc * cf.stage_stride;
         cf.ahead = pc > cf.rs && pc <= kMaxAhead * cf.rs && o + whole + std::min(want, (size_t)pc * 48) <= limit ? 1 : 0;
         if (cf.ahead) stage = std::max(stage, whole);
@@ -1420,11 +1423,12 @@ cudaError_t search_device(SearchDevice& out)
     return cudaSuccess;
 }
 
-// Fitted to single beams on GB300 (before the last 15 % came off every size: the choice needs
-// ratios only), us per level over survivors per block (v2, 20x20): one block 64: 5.8, 128: 6.4,
-// 256: 8.1, 384: 10.5, 512: 14.6, 1 024: 27.7, 2 048: 50.6; 2 blocks +1.9, 16 +3.8 (barriers);
-// lists of 50 / 100 jobs cost 1.4 / 2 times as much per survivor; v1 also writes the scored
-// children (1 024: 62.4).
+// Fitted to single beams on GB300 on an earlier build; the sizes have become faster since by unequal
+// factors, so these are estimates that choose among block counts, not times.  us per level over
+// survivors per block (v2, 20x20): one block 64: 5.8, 128: 6.4, 256: 8.1, 384: 10.5, 512: 14.6,
+// 1 024: 27.7, 2 048: 50.6; 2 blocks +1.9, 16 +3.8 (barriers); lists of 50 / 100 jobs cost 1.4 / 2
+// times as much per survivor; v1 also writes the scored children (1 024: 62.4).  The number of
+// machines is not in it.
 double search_level_us(int n, int K, bool v1, int C)
 {
     const double at[] = {64, 128, 256, 384, 512}, cost[] = {0, 0.7, 2.6, 5.2, 9.3}, slots[] = {0.9, 2.0, 4.8, 7.4, 10.0};

@@ -274,9 +274,9 @@ class Server:
     ``submit`` queues one solve and returns a ticket at once; the server admits queued
     requests while an in-flight slot and the memory budget allow, runs them concurrently
     and reuses plans by shape.  ``poll`` / ``wait`` return the result dict with
-    ``queue_ms`` and ``run_ms``.  Thread-safe.  ``cluster_inflight``: a request runs the
-    cluster select (K >= 4096) only when at most this many others are in flight at its
-    admission (0 = the device's SMs / 8, negative = never)."""
+    ``queue_ms`` and ``run_ms``.  Thread-safe.  ``cluster_inflight``: a request runs as
+    wide as the rule picks only when at most this many others are in flight at its admission,
+    else in the narrow form (0 = the device's SMs / 8, negative = always narrow)."""
 
     def __init__(self, device: int = 0, max_inflight: int = 0, memory_budget: int = 0, cluster_inflight: int = 0):
         self.lib = nat.load()

@@ -182,8 +182,9 @@ bsj_status bsj_plan_kernel_ms(const bsj_plan *plan, float *ms, int64_t *launches
    form runs the one-block routes on its first block.
    bsj_plan_select_routes: BSJ_ROUTE_* bits of the routes the last run took (OR over the
    plan's beams and levels; waits for the run).
-   With no flags and no forced k_step form the gpu modes run the resident search (m >= 2):
-   one launch for all levels, 1 to 16 thread blocks per beam.  What ran there:
+   With no flags and no forced k_step form the gpu modes run the resident search (m >= 2; but
+   v1 beams of K in (2048, 8192) whose children the level kernels write faster): one launch for
+   all levels, 1 to 16 thread blocks per beam.  What ran there:
      RESIDENT     some beam was searched by it;
      BLOCKS(c)    with c = 1, 2, 4, 8, 12 or 16 thread blocks;
      RECOUNT      a level's score bins were counted again over another range;
@@ -225,7 +226,7 @@ bsj_status bsj_plan_select_routes(bsj_plan *plan, uint32_t *routes);
 /* enable = 0: the narrow forms for this plan from its next run on, whatever K (a throughput
    choice: the cluster forms spend more SM time per level for their lower latency) -- the
    resident search with at most 4 thread blocks per beam (8 for wide beams of long lists,
-   where they cost hardly more SM time), and one block per beam for the level kernels'
+   where they cost hardly more SM time) and never more than the default form's, and one block per beam for the level kernels'
    selections; enable != 0 (the default): as wide as the rule picks.  Both forms' graphs are
    kept, so switching costs one capture per form; the results never depend on it.  The route
    flags above take precedence. */
@@ -292,9 +293,10 @@ bsj_status bsj_schedule_decode(const bsj_instance *inst, const int32_t *sequence
 typedef struct bsj_server bsj_server;
 typedef struct {
     int32_t max_inflight;    /* requests on the device at once; 0 = 32, at most 256 */
-    int32_t cluster_inflight; /* a request runs the cluster select (K >= 4096) only when at
-                                most this many others are in flight at its admission:
-                                0 = the device's SMs / 8, < 0 = never */
+    int32_t cluster_inflight; /* a request runs as wide as the rule picks only when at most this
+                                many others are in flight at its admission, else in the narrow
+                                form (bsj_plan_set_select_cluster): 0 = the device's SMs / 8,
+                                < 0 = always narrow */
     int64_t memory_budget;   /* device bytes held by running and idle plans; 0 = 3/4 of
                                 the free memory at creation */
 } bsj_server_config;

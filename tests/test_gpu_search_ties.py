@@ -57,7 +57,7 @@ def test_tied_levels_stay_resident(ctx, name, n, m, K):
 @pytest.mark.parametrize("mode,n,m", [("v2", 20, 3), ("clean", 30, 3), ("v1", 24, 4)])
 def test_wide_tied_levels_leave_one_block(ctx, mode, n, m):
     # a wide beam whose early levels fit no bins goes on with tie bins: it does not stay with one block
-    # (v1's stale slots bring back equal states in neighbouring ranks, which no bin tells apart)
+    # (a v1 beam's stale states score by their own number of operations, tie bins by the level's)
     mc, du = synthetic_instance(n, m, n + m)
     _, routes = _solve(ctx, mc, DURATIONS["small"](du).astype(np.int32), mode, 16384, 500000)
     assert "tie_bins" in routes and (mode == "v1" or "one_block" not in routes), routes
