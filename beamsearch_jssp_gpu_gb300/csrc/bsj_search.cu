@@ -198,11 +198,15 @@ constexpr int kTieMax = 1024;
 // a pass over the keys and two barriers.  384: 14.0 at 50x20 K=4096; 768 and 1 536: 13.5.
 constexpr int kRecountBin = 1536;
 constexpr int kMaxRecounts = 3;
-// Tie bins follow a level whose ranking was slow: one that sorted a block's window, or whose largest
-// group of equal scores had more than kTieSlow keys.  ms per call, 50x20 K=4096, durations
-// U[1, 99] | x 1 000: 384: 12.28 | 16.8, 192: 12.29 | 15.8, 96: 12.42 | 15.8.  They stay for 2, 4, ..
-// kTieStay levels, as long as linear bins fail each time between (a tie bin costs a division and a
-// pass over the keys: on every level of U[1, 99], 14.1).
+// Tie bins follow a level whose ranking was slow for its ties: one that sorted a block's window though
+// that spans few bins, or whose largest group of equal scores had more than kTieSlow keys.  ms per
+// call, 50x20 K=4096, durations U[1, 99] | x 1 000: 384: 12.28 | 16.8, 192: 12.29 | 15.8, 96: 12.42 |
+// 15.8.  They stay for 2, 4, .. kTieStay levels, as long as linear bins fail each time between (a tie
+// bin costs a division and a pass over the keys: on every level of U[1, 99], 14.1).  Not below
+// kTieBlocks blocks, whose pass takes 4 to 16 times as many keys per thread (levels that fit no bins
+// get tie bins there too): 256 mixed searches 2 590 -> 2 905 per second, 150 of 100x20 K=4096 497 ->
+// 452 ms; but 20 of 50x20 K=1024 on 4 blocks, durations 1 to 5: 20.3 ms without, 15.3 with.
+constexpr int kTieBlocks = 4;
 constexpr int kTieSlow = 192;
 constexpr int kTieStay = 64;
 
@@ -1094,7 +1098,7 @@ __global__ void __launch_bounds__(T, 1) k_search(StepArgs a, SearchCfg cf)
                     __syncthreads();
                     ok = s_tie <= kTieMax;
                 }
-                if (tid == 0 && !tie && (!ok || s_tie > kTieSlow)) s_slow = 1;
+                if (tid == 0 && !tie && C >= kTieBlocks && nb <= kSubBins && (!ok || s_tie > kTieSlow)) s_slow = 1;
                 if (ok) {
 #pragma unroll 1
                     for (int x = x0 + tid; x < x1; x += T) {
